@@ -131,20 +131,52 @@ __device__ __forceinline__ void issue_tile(const StreamSet& ss, long long t, uns
              bar, pol);
 }
 
-// Fill the partial last tile (elements [t*kTile, n)) with plain loads by the `nthr`
-// threads rank = 0..nthr-1; the rest of the stage is left as is (callers mask by index).
-__device__ __forceinline__ void fill_tail(const StreamSet& ss, long long t, long long n,
-                                          unsigned char* buf, int rank, int nthr) {
-  const long long first = t * kTile;
-  const long long valid = n - first;  // 0 < valid < kTile
-  for (int j = 0; j < ss.count; j++) {
-    const int tb = ss.tile_bytes[j];
-    // bytes of the valid prefix (bit streams round up to whole 32-bit words)
-    long long vb = (long long)tb * valid / kTile;
-    if ((long long)tb * valid % kTile) vb++;
-    if (tb < kTile) vb = ((vb + 3) / 4) * 4;
-    const unsigned char* src = ss.src[j] + (size_t)t * tb;
-    for (long long b = rank; b < vb; b += nthr) buf[ss.off[j] + b] = src[b];
+// Bytes of stream j's elements in the partial last tile (valid < kTile elements); bit
+// streams round up to whole 32-bit words.
+__device__ __forceinline__ uint32_t tail_bytes(const StreamSet& ss, int j, int valid) {
+  const uint32_t tb = (uint32_t)ss.tile_bytes[j];
+  uint32_t vb = (tb * (uint32_t)valid + kTile - 1) / kTile;
+  if (tb < (uint32_t)kTile) vb = (vb + 3) & ~3u;
+  return vb;
+}
+
+// Issue the partial last tile t (valid elements) into stage buffer `buf`, called by a whole
+// warp: the whole 16-byte words of each stream's valid prefix as one bulk copy, the rest (at
+// most 15 bytes a stream) by plain loads; the rest of the stage is left as is (callers mask
+// by index).  The caller arrives on the barrier afterwards: the phase then completes when the
+// bulk copies have landed.
+// Copied byte by byte by the warp, as one plain loop, the tail was 24 KB - 90 KB of dependent
+// single-byte loads: on a 333 x 333 grid (m = 5, FP64) a pass took 165-215 us, nearly all of
+// it the one CTA's tail, for 20-50 us of work.
+__device__ __forceinline__ void issue_tail(const StreamSet& ss, long long t, int valid,
+                                           unsigned char* buf, uint64_t* bar) {
+  const int lane = threadIdx.x & 31;
+  static_assert(kMaxStreams <= 32, "one lane per stream");
+  const uint32_t vb = lane < ss.count ? tail_bytes(ss, lane, valid) : 0;
+  const uint32_t whole = vb & ~15u;
+  const uint32_t sum = __reduce_add_sync(0xffffffffu, whole);
+  if (lane == 0)
+    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(sum)
+                 : "memory");
+  __syncwarp();
+  if (whole)
+    bulk_g2s(buf + ss.off[lane], ss.src[lane] + (size_t)t * ss.tile_bytes[lane], whole, bar,
+             l2_evict_first());
+  // two streams a step, 16 lanes each; every load is issued before the first store
+  unsigned char v[kMaxStreams / 2];
+#pragma unroll
+  for (int q = 0; q < kMaxStreams / 2; q++) {
+    const int j = 2 * q + (lane >> 4);
+    if (j >= ss.count) continue;
+    const uint32_t end = tail_bytes(ss, j, valid), k = (end & ~15u) + (lane & 15);
+    if (k < end) v[q] = ss.src[j][(size_t)t * ss.tile_bytes[j] + k];
+  }
+#pragma unroll
+  for (int q = 0; q < kMaxStreams / 2; q++) {
+    const int j = 2 * q + (lane >> 4);
+    if (j >= ss.count) continue;
+    const uint32_t end = tail_bytes(ss, j, valid), k = (end & ~15u) + (lane & 15);
+    if (k < end) buf[ss.off[j] + k] = v[q];
   }
 }
 
@@ -152,16 +184,15 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 
-// Stage buffer of tile t: full tiles by bulk copies (lanes of the calling warp issue the
-// copies of their streams), the partial last tile by plain loads of the warp's lanes and a
-// plain arrive.  Called by a whole warp.
+// Stage buffer of tile t, by bulk copies that the lanes of the calling warp issue; the partial
+// last tile's ragged ends by plain loads and a plain arrive.  Called by a whole warp.
 __device__ __forceinline__ void load_tile(const StreamSet& ss, long long t, long long n,
                                           unsigned char* buf, uint64_t* full) {
   const int lane = threadIdx.x & 31;
   if ((t + 1) * kTile <= n) {
     issue_tile(ss, t, buf, full);
   } else {
-    fill_tail(ss, t, n, buf, lane, 32);
+    issue_tail(ss, t, (int)(n - t * kTile), buf, full);
     __syncwarp();
     if (lane == 0) mbar_arrive(full);
   }
