@@ -30,43 +30,64 @@ namespace lbfgsb_b200 {
 extern thread_local std::string g_last_error;
 
 constexpr int kNoAllocThreads = 256;
-constexpr int kNoAllocPerCta = 4096;   // elements per CTA (16 per thread)
+constexpr int kNoAllocPerCta = 4096;   // elements per CTA at most (16 per thread)
 constexpr int kNoAllocRows = 8192;     // per-CTA maxima: at most 8192 CTAs
 constexpr long long kNoAllocMaxN = (long long)kNoAllocRows * kNoAllocPerCta;  // 2^25
+constexpr int kNoAllocWave = 8 * 148;  // CTAs resident on the chip together
 constexpr int kNoAllocMaxDevices = 64;
 
 // 64 KB of per-CTA maxima plus a 256-byte header holding the ticket.
 static __device__ __align__(256) unsigned long long g_projgr_scratch[32 + kNoAllocRows];
 
+// One launch of at most a few thousand variables is bound by latency (the loads, the ticket,
+// the fold), a large one by HBM.  kPer, the elements per thread, is chosen so that a small
+// call spreads over the SMs: with 16 each, in a loop, n = 65,536 ran on 16 CTAs and took
+// 16.3 us, one load round trip (two, for the bound that the sign of g selects) per element.
+// All loads of up to four elements are now issued together; both bounds are read (signs mix
+// within a 32-byte sector, so that one bound per element moves the same sectors).
+template <int kPer>
 __global__ void __launch_bounds__(kNoAllocThreads)
     k_projgr_noalloc(int n, const double* __restrict__ x, const double* __restrict__ g,
                      const int* __restrict__ nbd, const double* __restrict__ l,
                      const double* __restrict__ u, unsigned long long* scratch, double* out) {
   unsigned long long* ticket = scratch;
   unsigned long long* rows = scratch + 32;
-  const long long base = (long long)blockIdx.x * kNoAllocPerCta;
+  const long long base = (long long)blockIdx.x * (kPer * kNoAllocThreads) + threadIdx.x;
+  constexpr int kLoad = kPer < 4 ? kPer : 4;  // elements whose loads are in flight together
   double m = 0.0;
-  for (int k = threadIdx.x; k < kNoAllocPerCta; k += kNoAllocThreads) {
-    const long long i = base + k;
-    if (i >= n) break;
-    const double xi = x[i], gi = g[i];
-    const int nb = nbd[i];
-    double pg = gi;
-    if (nb != 0) {  // the reference's maxreal / minreal: (a > b) ? a : b, (a < b) ? a : b
-      if (gi < 0.0) {
-        if (nb >= 2) {
-          const double d = __dsub_rn(xi, u[i]);
-          pg = d > gi ? d : gi;
-        }
-      } else {
-        if (nb <= 2) {
-          const double d = __dsub_rn(xi, l[i]);
-          pg = d < gi ? d : gi;
+#pragma unroll 1
+  for (int k = 0; k < kPer; k += kLoad) {
+    double xi[kLoad], gi[kLoad], li[kLoad], ui[kLoad];
+    int nb[kLoad];
+#pragma unroll
+    for (int q = 0; q < kLoad; q++) {
+      const long long i = base + (long long)(k + q) * kNoAllocThreads;
+      const bool in = i < n;
+      xi[q] = in ? x[i] : 0.0;
+      gi[q] = in ? g[i] : 0.0;  // g = 0, nbd = 0 adds |0|
+      nb[q] = in ? nbd[i] : 0;
+      li[q] = in ? l[i] : 0.0;
+      ui[q] = in ? u[i] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < kLoad; q++) {
+      double pg = gi[q];
+      if (nb[q] != 0) {  // the reference's maxreal / minreal: (a > b) ? a : b, (a < b) ? a : b
+        if (gi[q] < 0.0) {
+          if (nb[q] >= 2) {
+            const double d = __dsub_rn(xi[q], ui[q]);
+            pg = d > gi[q] ? d : gi[q];
+          }
+        } else {
+          if (nb[q] <= 2) {
+            const double d = __dsub_rn(xi[q], li[q]);
+            pg = d < gi[q] ? d : gi[q];
+          }
         }
       }
+      const double a = fabs(pg);
+      m = a > m ? a : m;
     }
-    const double a = fabs(pg);
-    m = a > m ? a : m;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -162,8 +183,18 @@ extern "C" int lbfgsb_b200_projgr_noalloc_f64(int n, const double* x, const doub
   if (n == 0) {
     e = cudaMemsetAsync(sbgnrm, 0, sizeof(double), s);  // the reference's sbgnrm = 0
   } else {
-    const int rows = (int)(((long long)n + kNoAllocPerCta - 1) / kNoAllocPerCta);
-    k_projgr_noalloc<<<rows, kNoAllocThreads, 0, s>>>(n, x, g, nbd, l, u, scratch, sbgnrm);
+    // one element a thread up to about eight CTAs per SM, then four, then sixteen (the most
+    // rows the scratch holds)
+    auto launch = [&](auto kernel, int per_cta) {
+      const int rows = (int)(((long long)n + per_cta - 1) / per_cta);
+      kernel<<<rows, kNoAllocThreads, 0, s>>>(n, x, g, nbd, l, u, scratch, sbgnrm);
+    };
+    if (n <= kNoAllocWave * kNoAllocThreads)
+      launch(k_projgr_noalloc<1>, kNoAllocThreads);
+    else if (n <= 4 * kNoAllocWave * kNoAllocThreads)
+      launch(k_projgr_noalloc<4>, 4 * kNoAllocThreads);
+    else
+      launch(k_projgr_noalloc<16>, kNoAllocPerCta);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) {
