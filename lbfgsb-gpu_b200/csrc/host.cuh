@@ -255,14 +255,17 @@ static void walk_buffers(Workspace<R, H, S>& w, Ctx<R, H, S>& c, size_t N) {
   c.wl_t = w.wl_t;
   c.wl_i = w.wl_i;
   c.wl_n = w.wl_n;
-  c.wsc = w.template alloc<WalkScratch>(1);
+  c.wsc = reinterpret_cast<WalkScratch*>(w.template alloc<unsigned char>(walk_scratch_bytes<S>((int)N)));
 }
 
 // Grid of the cooperative walk: CTAs that are all resident at once (one per SM at most).
 template <typename R, typename H, typename S>
 static int walk_coop_grid() {
   int per_sm = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk_coop<R, H, S>, kWalkThreads, 0));
+  CK(cudaFuncSetAttribute(k_walk_coop<R, H, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                          (int)sizeof(WalkCoop<S>)));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk_coop<R, H, S>, kWalkThreads,
+                                                   sizeof(WalkCoop<S>)));
   if (per_sm < 1) throw CudaFailure{cudaErrorCooperativeLaunchTooLarge, "k_walk_coop occupancy", __LINE__};
   return device_sms();
 }
@@ -276,7 +279,7 @@ static void launch_walk_coop(const Ctx<R, H, S>& c, const R* x, const R* g, int 
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kWalkThreads);
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = sizeof(WalkCoop<S>);
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;

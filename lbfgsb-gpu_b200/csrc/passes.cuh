@@ -37,19 +37,17 @@
 namespace lbfgsb_b200 {
 
 // Scratch of the cooperative breakpoint walk (walk.cuh, k_walk_coop): its grid barrier,
-// the radix-select histograms (three, used in rotation), and the selected chunk.
-constexpr int kWalkChunk = 1024;  // breakpoints selected and sorted at a time
+// and the radix-select histograms (three, used in rotation).
+constexpr int kWalkChunk = 1024;  // breakpoints the other walks select and sort at a time
 struct WalkScratch {
   unsigned int bar;      // grid-barrier arrivals; zero before each launch
   unsigned int chunk_n;  // keys of the selected chunk
   int done;              // the walk has ended
-  int cnt;               // keys in the chunk just walked
   unsigned long long last_hi;  // largest key walked so far
   unsigned int last_lo;
   unsigned int pad;
   unsigned int hist[3][256];
-  unsigned long long chunk_hi[kWalkChunk];
-  unsigned int chunk_lo[kWalkChunk];
+  // the chunk's records follow (walk.cuh)
 };
 
 template <typename R, typename H, typename S>

@@ -11,10 +11,10 @@
 //   walk     the chunk is sorted in shared memory (bitonic), each candidate's row of W,
 //            M*wbp and wbp'M wbp are formed in parallel, and one thread walks the chunk in
 //            key order with the reference's recurrence for f', f'', c and p.
-// Two forms: k_walk_coop (single-instance solves) lists and selects with the whole grid, a
-// cooperative launch with a bounded grid barrier, and walks in CTA 0; k_walk (one CTA per
-// instance, used by batched solves, with k_walk_gather before it) does everything in one
-// CTA.  Breakpoints with equal t are passed in increasing variable index (the heap's order
+// Two forms: k_walk_coop (single-instance solves) lists, selects, sorts and prepares with the
+// whole grid, a cooperative launch with a bounded grid barrier, and walks in CTA 0 as a
+// pipeline of warps; k_walk (one CTA per instance, used by batched solves, with k_walk_gather
+// before it) does everything in one CTA as described above.  Breakpoints with equal t are passed in increasing variable index (the heap's order
 // among exact ties is an artefact of its layout).
 #pragma once
 
@@ -471,9 +471,389 @@ __device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned int& ta
   return s_ok != 0;
 }
 
-// Lists the breakpoints with the whole grid, selects each chunk with the whole grid
-// (histograms in global memory, the same digit decided redundantly by every CTA) and walks
-// it in CTA 0.  wsc->bar and *wl_n are zero at launch.
+// The cooperative walk takes the breakpoints in chunks of up to kWalkRows keys.  For each
+// chunk the whole grid selects it (histograms in global memory, the same digit decided
+// redundantly by every CTA), sorts it (pieces of kPiece keys, one CTA each; a key's rank is
+// its position in its piece plus its lower bounds in the others) and prepares each key's
+// record: its row times its step, M*wbp and wbp'M wbp.  CTA 0 then walks the records.
+//
+// The walk is the reference's recurrence with its operations unchanged, cut into the chains
+// that depend on one another, each run by its own warp over sub-batches of kSub keys one
+// sub-batch behind the warp that feeds it:
+//   scan    p += (-dibp) wbp and c += dt p need no f' or f'': one lane per component, one
+//           dependent addition a key;
+//   dots    wbp'M c and wbp'M p, one thread per key, and the terms of f' and f'';
+//   chain   f' and f'': three or four dependent additions each a key, on one thread (the
+//           walk's rate: the reference's order of these additions is kept); sum of dt beside;
+//   test    dtm = -f'/f'' against the next breakpoint's distance, one lane per key.
+// The keys after the one where the walk ends are worked on in vain (at most four sub-batches).
+//
+// One thread walking key by key, with 64 rows of M*wbp prepared at a time by 64 threads,
+// took 0.46-0.52 us a breakpoint (n = 512^2, 217,112 breakpoints in one walk: 112 ms).
+constexpr int kWalkRows = 8192;       // breakpoints of a chunk at most
+constexpr int kWalkFirst = 1024;      // of the first chunk (most walks are short); then doubled
+constexpr int kPiece = kWalkThreads;  // keys sorted together
+constexpr int kMaxPieces = kWalkRows / kPiece;
+constexpr int kSub = 128;             // keys of a pipeline step
+constexpr int kRow = 2 * kMaxM;
+
+// The records of a chunk, after the WalkScratch header (walk_scratch_bytes in all).
+template <typename S>
+struct WalkRecords {
+  unsigned long long *raw_hi, *hi;  // keys as extracted (then sorted by piece), keys in order
+  S *e, *v;                         // rows of kRow: (-dibp) wbp, M wbp
+  S *dibp, *zibp, *wmw;
+  unsigned int *raw_lo, *lo;
+};
+__host__ __device__ inline int walk_rows(int n) {
+  return n < kWalkRows ? (n + kPiece - 1) / kPiece * kPiece : kWalkRows;
+}
+template <typename S>
+__host__ __device__ inline size_t walk_scratch_bytes(int n) {
+  return (sizeof(WalkScratch) + 255) / 256 * 256 +
+         (size_t)walk_rows(n) * (2 * 8 + 2 * 4 + (2 * kRow + 3) * sizeof(S));
+}
+template <typename S>
+__device__ __forceinline__ WalkRecords<S> walk_records(WalkScratch* ws, int n) {
+  const size_t rows = (size_t)walk_rows(n);
+  WalkRecords<S> r;
+  r.raw_hi = reinterpret_cast<unsigned long long*>(reinterpret_cast<unsigned char*>(ws) +
+                                                   (sizeof(WalkScratch) + 255) / 256 * 256);
+  r.hi = r.raw_hi + rows;
+  r.e = reinterpret_cast<S*>(r.hi + rows);
+  r.v = r.e + rows * kRow;
+  r.dibp = r.v + rows * kRow;
+  r.zibp = r.dibp + rows;
+  r.wmw = r.zibp + rows;
+  r.raw_lo = reinterpret_cast<unsigned int*>(r.wmw + rows);
+  r.lo = r.raw_lo + rows;
+  return r;
+}
+
+// Dynamic shared memory of k_walk_coop.
+template <typename S>
+struct WalkCoop {
+  unsigned long long k_hi[kPiece];
+  unsigned int k_lo[kPiece];
+  unsigned int hist[256];
+  S sy[kMaxM * kMaxM], wt[kMaxM * kMaxM];
+  S wbp[kBatch][kRow + 1], bv[kBatch][kRow + 1], work[kBatch][kMaxM + 1];
+  // CTA 0's pipeline; buffers are indexed by sub-batch modulo their count
+  S e[2][kSub][kRow];
+  S p[2][kSub][kRow + 1], c[2][kSub][kRow + 1];  // p before, c after each key
+  S dt[8][kSub];
+  S a1[2][kSub], a2[2][kSub], a3[2][kSub], b1[2][kSub], b2[2][kSub], b3[2][kSub];
+  S f1s[2][kSub], f2s[2][kSub], ts[2][kSub];     // after each key
+  S ckp[kWalkRows / kSub][kRow], ckc[kWalkRows / kSub][kRow];  // p, c before each sub-batch
+  S f1, f2, dtm, tsum, tj;                       // before the next key to be tested
+  int nleft, nint, all_fixed, done, stop, passed, info;
+};
+
+// Sorts the kPiece keys of sm.k_hi / k_lo (all threads of the CTA, one key each).
+template <typename S>
+__device__ void sort_piece(WalkCoop<S>& sm) {
+  const int e = (int)threadIdx.x;
+  for (int size = 2; size <= kPiece; size <<= 1) {
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      __syncthreads();
+      const int p = e ^ stride;
+      if (p > e) {
+        const bool up = (e & size) == 0;
+        const Key96 a{sm.k_hi[e], sm.k_lo[e]}, b{sm.k_hi[p], sm.k_lo[p]};
+        if (key_less(b, a) == up) {
+          sm.k_hi[e] = b.hi;
+          sm.k_lo[e] = b.lo;
+          sm.k_hi[p] = a.hi;
+          sm.k_lo[p] = a.lo;
+        }
+      }
+    }
+  }
+  __syncthreads();
+}
+
+// Rank of key k (position q of the pieces, each sorted) among the chunk's cnt keys.
+template <typename S>
+__device__ __forceinline__ int chunk_rank(const WalkRecords<S>& rec, const Key96& k, int q, int cnt) {
+  int lb[kMaxPieces];
+#pragma unroll
+  for (int pc = 0; pc < kMaxPieces; pc++) lb[pc] = 0;
+  const int own = q / kPiece;
+  for (int step = kPiece; step > 0; step >>= 1) {
+#pragma unroll
+    for (int pc = 0; pc < kMaxPieces; pc++) {
+      const int base = pc * kPiece, at = lb[pc] + step;
+      if (pc != own && at <= kPiece && base + at <= cnt) {
+        const Key96 o{__ldcg(&rec.raw_hi[base + at - 1]), __ldcg(&rec.raw_lo[base + at - 1])};
+        if (key_less(o, k)) lb[pc] = at;
+      }
+    }
+  }
+  int r = q - own * kPiece;
+#pragma unroll
+  for (int pc = 0; pc < kMaxPieces; pc++) r += lb[pc];
+  return r;
+}
+
+// sdot of two rows of col2 values, a in registers.
+template <typename S>
+__device__ __forceinline__ S row_dot(const S* b, const S (&a)[kRow], int col2) {
+  S r = 0;
+#pragma unroll
+  for (int g = 0; g < kRow; g += 4) {
+    if (g + 4 <= col2) {
+      r += b[g] * a[g] + b[g + 1] * a[g + 1] + b[g + 2] * a[g + 2] + b[g + 3] * a[g + 3];
+    } else if (g + 2 <= col2) {
+      r += b[g] * a[g];
+      r += b[g + 1] * a[g + 1];
+    }
+  }
+  return r;
+}
+
+// CTA 0: walks the cnt records in order (all threads).  sm.f1 .. sm.nint carry the walk from
+// chunk to chunk; st->p and st->c hold p and c.  Sets sm.done when the walk has ended.
+template <typename R, typename H, typename S>
+__device__ void walk_records_in_order(const Ctx<R, H, S>& c, const WalkRecords<S>& rec, int cnt,
+                                      WalkCoop<S>& sm) {
+  DevState<S>* st = c.st;
+  const int col2 = 2 * st->col, nbreak = st->nbreak, bnded = st->bnded, n = st->n;
+  const S theta = st->theta, floor2 = (S)(5e-16 * (double)st->f2org);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nsub = (cnt + kSub - 1) / kSub;
+  auto t_of = [&](int k) { return (S)__longlong_as_double((long long)__ldcg(&rec.hi[k])); };
+  auto stage = [&](int b, int tid, int nt) {
+    const int base = b * kSub, nk = cnt - base < kSub ? cnt - base : kSub;
+    for (int q = tid; q < nk; q += nt) {
+      const int k = base + q;
+      sm.dt[b & 7][q] = t_of(k) - (k > 0 ? t_of(k - 1) : sm.tj);
+    }
+    if (col2 > 0)
+      for (int q = tid; q < nk * kRow; q += nt)
+        (&sm.e[b & 1][0][0])[q] = __ldcg(&rec.e[(size_t)base * kRow + q]);
+  };
+  S pj = 0, cj = 0;  // warp 0: component `lane` of p and c
+  if (warp == 0 && lane < col2) {
+    pj = st->p[lane + 1];
+    cj = st->c[lane + 1];
+  }
+  if (threadIdx.x == 0) {
+    sm.stop = 0;
+    sm.passed = cnt;
+  }
+  stage(0, threadIdx.x, blockDim.x);
+  __syncthreads();
+  for (int s = 0; s < nsub + 3; s++) {
+    if (warp >= 8) {
+      if (s + 1 < nsub) stage(s + 1, (int)threadIdx.x - 256, (int)blockDim.x - 256);
+    } else if (warp == 0) {
+      if (s < nsub && col2 > 0 && lane < kRow) {
+        const int b = s & 1, nk = cnt - s * kSub < kSub ? cnt - s * kSub : kSub;
+        const S* dt = sm.dt[s & 7];
+        sm.ckp[s][lane] = pj;
+        sm.ckc[s][lane] = cj;
+        int q = 0;
+        for (; q + 8 <= nk; q += 8) {
+          S d[8], e[8];
+#pragma unroll
+          for (int u = 0; u < 8; u++) {
+            d[u] = dt[q + u];
+            e[u] = sm.e[b][q + u][lane];
+          }
+#pragma unroll
+          for (int u = 0; u < 8; u++) {
+            sm.p[b][q + u][lane] = pj;
+            cj += d[u] * pj;
+            sm.c[b][q + u][lane] = cj;
+            pj += e[u];
+          }
+        }
+        for (; q < nk; q++) {
+          sm.p[b][q][lane] = pj;
+          cj += dt[q] * pj;
+          sm.c[b][q][lane] = cj;
+          pj += sm.e[b][q][lane];
+        }
+      }
+    } else if (warp >= 4) {
+      const int b = s - 1, q = (int)threadIdx.x - 128;
+      if (b >= 0 && b < nsub && b * kSub + q < cnt) {
+        const int k = b * kSub + q, o = b & 1;
+        const S dibp = __ldcg(&rec.dibp[k]), zibp = __ldcg(&rec.zibp[k]);
+        const S dibp2 = dibp * dibp;
+        sm.a1[o][q] = dibp2;
+        sm.a2[o][q] = theta * dibp * zibp;
+        sm.b1[o][q] = theta * dibp2;
+        if (col2 > 0) {
+          S v[kRow];
+#pragma unroll
+          for (int j = 0; j < kRow; j++) v[j] = j < col2 ? __ldcg(&rec.v[(size_t)k * kRow + j]) : S(0);
+          const S wmw = __ldcg(&rec.wmw[k]);
+          const S wmc = row_dot(sm.c[o][q], v, col2), wmp = row_dot(sm.p[o][q], v, col2);
+          sm.a3[o][q] = dibp * wmc;
+          sm.b2[o][q] = (S)2.0 * dibp * wmp;
+          sm.b3[o][q] = dibp2 * wmw;
+        }
+      }
+    } else if (warp == 1) {
+      const int b = s - 2;
+      if (lane == 0 && b >= 0 && b < nsub) {
+        const int o = b & 1, nk = cnt - b * kSub < kSub ? cnt - b * kSub : kSub;
+        const S* dt = sm.dt[b & 7];
+        // f' and f'' after the last key of the sub-batch before
+        S f1 = b > 0 ? sm.f1s[o ^ 1][kSub - 1] : sm.f1, f2 = b > 0 ? sm.f2s[o ^ 1][kSub - 1] : sm.f2;
+        constexpr int U = 4;
+        int q = 0;
+        for (; q + U <= nk; q += U) {
+          S d[U], a1[U], a2[U], a3[U], b1[U], b2[U], b3[U];
+#pragma unroll
+          for (int u = 0; u < U; u++) {
+            d[u] = dt[q + u];
+            a1[u] = sm.a1[o][q + u];
+            a2[u] = sm.a2[o][q + u];
+            b1[u] = sm.b1[o][q + u];
+            a3[u] = sm.a3[o][q + u];
+            b2[u] = sm.b2[o][q + u];
+            b3[u] = sm.b3[o][q + u];
+          }
+          // without the lower limit of f'', which hardly ever acts; if it does, once more
+          const S g1 = f1, g2 = f2;
+          bool low = false;
+          S r1[U], r2[U];
+#pragma unroll
+          for (int u = 0; u < U; u++) {
+            f1 = f1 + d[u] * f2 + a1[u] - a2[u];
+            f2 = f2 - b1[u];
+            if (col2 > 0) {
+              f1 = f1 + a3[u];
+              f2 = f2 + b2[u] - b3[u];
+            }
+            low = low || floor2 > f2;
+            r1[u] = f1;
+            r2[u] = f2;
+          }
+          if (low) {
+            f1 = g1;
+            f2 = g2;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+              f1 = f1 + d[u] * f2 + a1[u] - a2[u];
+              f2 = f2 - b1[u];
+              if (col2 > 0) {
+                f1 = f1 + a3[u];
+                f2 = f2 + b2[u] - b3[u];
+              }
+              f2 = smax(floor2, f2);
+              r1[u] = f1;
+              r2[u] = f2;
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < U; u++) {
+            sm.f1s[o][q + u] = r1[u];
+            sm.f2s[o][q + u] = r2[u];
+          }
+        }
+        for (; q < nk; q++) {
+          f1 = f1 + dt[q] * f2 + sm.a1[o][q] - sm.a2[o][q];
+          f2 = f2 - sm.b1[o][q];
+          if (col2 > 0) {
+            f1 = f1 + sm.a3[o][q];
+            f2 = f2 + sm.b2[o][q] - sm.b3[o][q];
+          }
+          f2 = smax(floor2, f2);
+          sm.f1s[o][q] = f1;
+          sm.f2s[o][q] = f2;
+        }
+      }
+    } else if (warp == 2) {
+      const int b = s - 2;
+      if (lane == 0 && b >= 0 && b < nsub) {
+        const int o = b & 1, nk = cnt - b * kSub < kSub ? cnt - b * kSub : kSub;
+        const S* dt = sm.dt[b & 7];
+        S ts = b > 0 ? sm.ts[o ^ 1][kSub - 1] : sm.tsum;
+#pragma unroll 4
+        for (int q = 0; q < nk; q++) {
+          ts = ts + dt[q];
+          sm.ts[o][q] = ts;
+        }
+      }
+    } else {  // warp 3
+      const int b = s - 3;
+      if (b >= 0) {
+        const int o = b & 1, base = b * kSub, nk = cnt - base < kSub ? cnt - base : kSub;
+        const S* dt = sm.dt[b & 7];
+        int hit = -1;
+        for (int r = 0; r < nk && hit < 0; r += 32) {
+          const int q = r + lane;
+          bool ends = false;
+          if (q < nk) {
+            const S dtm = q == 0 ? sm.dtm : -sm.f1s[o][q - 1] / sm.f2s[o][q - 1];
+            ends = dtm < dt[q];
+          }
+          const unsigned bal = __ballot_sync(0xffffffffu, ends);
+          if (bal) hit = r + __ffs(bal) - 1;
+        }
+        __syncwarp();
+        if (lane == 0) {
+          const int q = hit >= 0 ? hit : nk;  // the sub-batch's keys passed
+          const bool last = hit < 0 && sm.nleft - (base + nk) == 0;
+          sm.tj = t_of(hit >= 0 ? base + hit : base + nk - 1);
+          // every variable has reached its bound: the last key moves c and sum dt only
+          const bool fixed = last && nbreak == n;
+          const int f = fixed ? q - 1 : q;
+          if (q > 0) sm.tsum = sm.ts[o][q - 1];
+          if (f > 0) {
+            sm.f1 = sm.f1s[o][f - 1];
+            sm.f2 = sm.f2s[o][f - 1];
+            sm.dtm = -sm.f1 / sm.f2;
+          }
+          if (fixed) {
+            sm.dtm = dt[q - 1];
+            sm.all_fixed = 1;
+          } else if (last && bnded) {
+            sm.f1 = 0;
+            sm.f2 = 0;
+            sm.dtm = 0;
+          }
+          if (hit >= 0) {
+            sm.stop = 1;
+            sm.passed = base + hit;
+          }
+          if (hit >= 0 || last) sm.done = 1;
+        }
+      }
+    }
+    __syncthreads();
+    if (sm.stop) break;
+  }
+  const int passed = sm.passed;
+  if (warp == 0 && lane < col2) {
+    if (sm.stop || sm.all_fixed) {
+      // p and c where the walk ended, from the start of that sub-batch
+      const int b = sm.stop ? passed / kSub : (cnt - 1) / kSub;
+      pj = sm.ckp[b][lane];
+      cj = sm.ckc[b][lane];
+      for (int k = b * kSub; k < passed; k++) {
+        cj += sm.dt[b & 7][k - b * kSub] * pj;
+        if (!(sm.all_fixed && k == cnt - 1)) pj += __ldcg(&rec.e[(size_t)k * kRow + lane]);
+      }
+    }
+    st->p[lane + 1] = pj;
+    st->c[lane + 1] = cj;
+  }
+  for (int k = threadIdx.x; k < passed; k += blockDim.x)
+    c.code[(int)__ldcg(&rec.lo[k])] =
+        (int8_t)(__ldcg(&rec.dibp[k]) > S(0) ? IW_WALK_UPP : IW_WALK_LOW);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    sm.nleft -= passed;
+    sm.nint += passed - sm.all_fixed;
+  }
+}
+
+// Lists the breakpoints with the whole grid and walks them chunk by chunk.  wsc->bar and
+// *wl_n are zero at launch.
 template <typename R, typename H, typename S>
 __global__ void __launch_bounds__(kWalkThreads) k_walk_coop(Ctx<R, H, S> c, const R* __restrict__ x,
                                                             const R* __restrict__ g) {
@@ -484,70 +864,99 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_coop(Ctx<R, H, S> c, cons
     g = c.G[st->gr[0]];
   }
   if (st->gcp_state != GCP_WALK) return;
+  extern __shared__ __align__(128) unsigned char dyn[];
+  WalkCoop<S>& sm = *reinterpret_cast<WalkCoop<S>*>(dyn);
   WalkScratch* ws = c.wsc;
+  const int col = st->col, col2 = 2 * col;
+  const S theta = st->theta;
+  for (int k = threadIdx.x; k < kMaxM * kMaxM; k += blockDim.x) {
+    sm.sy[k] = st->sy[k];
+    sm.wt[k] = st->wt[k];
+  }
+  if (threadIdx.x == 0) {
+    // a zero on the factor's diagonal fails every M*wbp (the driver resets the memory)
+    sm.info = 0;
+    for (int j = col; j >= 1; j--)
+      if (LB_AT(st->wt, kMaxM, j, j) == S(0)) sm.info = j;
+  }
+  __syncthreads();
+  const bool lead = blockIdx.x == 0;
   unsigned int target = 0;
+  if (sm.info != 0) {
+    // the other CTAs may still read internal_fail at the top: written after the barrier
+    if (!grid_barrier(&ws->bar, target)) {
+      if (threadIdx.x == 0) atomicExch(&st->device_error, 1);
+      return;
+    }
+    if (lead && threadIdx.x == 0) st->internal_fail = sm.info;
+    return;
+  }
   auto fail = [&]() {
     if (threadIdx.x == 0) atomicExch(&st->device_error, 1);
   };
-  __shared__ WalkSmem<S> sm;
-  const bool lead = blockIdx.x == 0;
+  const WalkRecords<S> rec = walk_records<S>(ws, c.n);
   if (lead) {
     for (int b = threadIdx.x; b < 256; b += blockDim.x) ws->hist[0][b] = 0;
-    if (threadIdx.x == 0) ws->chunk_n = 0;
+    if (threadIdx.x == 0) {
+      ws->chunk_n = 0;
+      const WalkCarry<S> w = walk_start(st);
+      sm.f1 = w.f1;
+      sm.f2 = w.f2;
+      sm.dtm = w.dtm;
+      sm.tsum = w.tsum;
+      sm.tj = w.tj;
+      sm.nleft = w.nleft;
+      sm.nint = w.nint;
+      sm.all_fixed = 0;
+      sm.done = 0;
+    }
   }
   gather_breakpoints<R, H, S>(c, cta_here(), blockDim.x, x, g);
   if (!grid_barrier(&ws->bar, target)) return fail();
   const long long L = (long long)*(volatile unsigned int*)c.wl_n;
   const H *Y[kMaxM], *Sl[kMaxM];
-  WalkCarry<S> w{};
-  if (lead) {
-    ring_ptrs(st, c.wy, c.ld, Y);
-    ring_ptrs(st, c.ws, c.ld, Sl);
-    if (threadIdx.x == 0) {
-      w = walk_start(st);
-      sm.done = 0;
-      sm.info = 0;
-    }
-  }
+  ring_ptrs(st, c.wy, c.ld, Y);
+  ring_ptrs(st, c.ws, c.ld, Sl);
   const long long stride = (long long)gridDim.x * blockDim.x;
-  const long long e0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long e0 = (long long)blockIdx.x * blockDim.x;
+  const int lane = threadIdx.x & 31;
   bool first_round = true;
   Key96 last{0ull, 0u};
   long long consumed = 0;
+  int want = kWalkFirst < walk_rows(c.n) ? kWalkFirst : walk_rows(c.n);
   int hb = 0;  // the histogram buffer of the next level (rotating over three)
-  __shared__ unsigned int s_hist[256];
   while (true) {
     const long long remaining = L - consumed;
     Key96 thr{~0ull, ~0u};
-    if (remaining > kChunk) {
+    if (remaining > want) {
       Key96 prefix{0ull, 0u};
-      long long kk = kChunk, taken = 0;
+      long long kk = want, taken = 0;
       for (int level = 0; level < 12; level++) {
         unsigned int* h = ws->hist[hb];
         // the buffer after this one was last read two levels ago, before the previous
         // barrier: clear it for the next level
         if (lead)
           for (int b = threadIdx.x; b < 256; b += blockDim.x) ws->hist[(hb + 1) % 3][b] = 0;
-        for (int b = threadIdx.x; b < 256; b += blockDim.x) s_hist[b] = 0;
+        for (int b = threadIdx.x; b < 256; b += blockDim.x) sm.hist[b] = 0;
         __syncthreads();
-        for (long long e = e0; e < L; e += stride) {
+        for (long long e = e0 + threadIdx.x; e < L; e += stride) {
           const Key96 k = make_key(c.wl_t[e], c.wl_i[e]);
           if (!first_round && !key_less(last, k)) continue;
           if (!key_prefix_eq(k, prefix, level)) continue;
-          atomicAdd(&s_hist[key_digit(k, level)], 1u);
+          atomicAdd(&sm.hist[key_digit(k, level)], 1u);
         }
         __syncthreads();
         for (int b = threadIdx.x; b < 256; b += blockDim.x)
-          if (s_hist[b]) atomicAdd(&h[b], s_hist[b]);
+          if (sm.hist[b]) atomicAdd(&h[b], sm.hist[b]);
         if (!grid_barrier(&ws->bar, target)) return fail();
-        for (int b = threadIdx.x; b < 256; b += blockDim.x) s_hist[b] = __ldcg(&h[b]);
+        for (int b = threadIdx.x; b < 256; b += blockDim.x) sm.hist[b] = __ldcg(&h[b]);
         __syncthreads();
         hb = (hb + 1) % 3;
         int d;
         long long cum;
         bool stop;
-        select_level(s_hist, taken, kk, kChunkMin, d, cum, stop);
-        __syncthreads();  // every thread has read s_hist before the next level clears it
+        select_level(sm.hist, taken, kk, want / 4, d, cum, stop);
+        __syncthreads();  // every thread has read the histogram before the next level clears it
         key_set_digit(prefix, level, d);
         if (stop) {
           prefix = key_prev(prefix);
@@ -559,47 +968,122 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_coop(Ctx<R, H, S> c, cons
       thr = prefix;
     }
     // extract the chunk: keys in (last, thr]
-    for (long long e = e0; e < L; e += stride) {
-      const Key96 k = make_key(c.wl_t[e], c.wl_i[e]);
-      if (!first_round && !key_less(last, k)) continue;
-      if (key_less(thr, k)) continue;
-      const unsigned int pos = atomicAdd(&ws->chunk_n, 1u);
-      if (pos < (unsigned int)kChunk) {
-        ws->chunk_hi[pos] = k.hi;
-        ws->chunk_lo[pos] = k.lo;
+    for (long long e1 = e0; e1 < L; e1 += stride) {
+      const long long e = e1 + threadIdx.x;
+      Key96 k{0ull, 0u};
+      bool take = false;
+      if (e < L) {
+        k = make_key(c.wl_t[e], c.wl_i[e]);
+        take = (first_round || key_less(last, k)) && !key_less(thr, k);
+      }
+      const unsigned mask = __ballot_sync(0xffffffffu, take);
+      if (mask == 0) continue;
+      unsigned int start = 0;
+      if (lane == 0) start = atomicAdd(&ws->chunk_n, (unsigned int)__popc(mask));
+      start = __shfl_sync(0xffffffffu, start, 0);
+      const unsigned int pos = start + __popc(mask & ((1u << lane) - 1u));
+      if (take && pos < (unsigned int)walk_rows(c.n)) {
+        rec.raw_hi[pos] = k.hi;
+        rec.raw_lo[pos] = k.lo;
       }
     }
     if (!grid_barrier(&ws->bar, target)) return fail();
-    if (lead) {
-      const unsigned int n_sel = __ldcg(&ws->chunk_n);
-      const int cnt = n_sel < (unsigned int)kChunk ? (int)n_sel : kChunk;
-      for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-        sm.k_hi[e] = __ldcg(&ws->chunk_hi[e]);
-        sm.k_lo[e] = __ldcg(&ws->chunk_lo[e]);
+    const unsigned int n_sel = __ldcg(&ws->chunk_n);
+    const int cnt = n_sel < (unsigned int)want ? (int)n_sel : want;
+    if (cnt == 0) break;
+    // sort the pieces
+    for (int pc = blockIdx.x; pc * kPiece < cnt; pc += gridDim.x) {
+      const int q = pc * kPiece + (int)threadIdx.x;
+      sm.k_hi[threadIdx.x] = q < cnt ? __ldcg(&rec.raw_hi[q]) : ~0ull;
+      sm.k_lo[threadIdx.x] = q < cnt ? __ldcg(&rec.raw_lo[q]) : ~0u;
+      sort_piece(sm);
+      if (q < cnt) {
+        rec.raw_hi[q] = sm.k_hi[threadIdx.x];
+        rec.raw_lo[q] = sm.k_lo[threadIdx.x];
       }
       __syncthreads();
-      walk_chunk<R, H, S>(c, x, g, Y, Sl, sm, cnt, w);
-      if (threadIdx.x == 0) {
-        ws->chunk_n = 0;
-        ws->cnt = cnt;
-        ws->done = sm.done;
-        if (cnt > 0) {
-          ws->last_hi = sm.k_hi[cnt - 1];
-          ws->last_lo = sm.k_lo[cnt - 1];
+    }
+    if (!grid_barrier(&ws->bar, target)) return fail();
+    if (lead && threadIdx.x == 0) ws->chunk_n = 0;
+    // rank every key and prepare its record there, the keys spread over the CTAs
+    for (int q0 = 0; q0 < cnt; q0 += kBatch * (int)gridDim.x) {
+      const int q = q0 + (int)threadIdx.x * (int)gridDim.x + (int)blockIdx.x;
+      if (threadIdx.x >= kBatch || q >= cnt) continue;
+      const Key96 k{__ldcg(&rec.raw_hi[q]), __ldcg(&rec.raw_lo[q])};
+      const int i = (int)k.lo;
+      S* wbp = sm.wbp[threadIdx.x];
+      S* v = sm.bv[threadIdx.x];
+      const R xi = x[i], gi = g[i];
+#pragma unroll
+      for (int j = 0; j < kMaxM; j++)
+        if (j < col) {
+          wbp[1 + j] = (S)HistTraits<H>::load(Y[j] + i);
+          wbp[1 + col + j] = theta * (S)HistTraits<H>::load(Sl[j] + i);
+        }
+      const int r = chunk_rank(rec, k, q, cnt);
+      const R dibp = -gi;
+      const R zibp = (dibp > R(0)) ? rsub(c.u[i], xi) : rsub(c.l[i], xi);
+      rec.hi[r] = k.hi;
+      rec.lo[r] = k.lo;
+      rec.dibp[r] = (S)dibp;
+      rec.zibp[r] = (S)zibp;
+      if (col > 0) {
+        int info = 0;
+        sbmv(sm.sy, sm.wt, col, wbp, v, &info, sm.work[threadIdx.x]);
+        rec.wmw[r] = sdot(&wbp[1], 1, &v[1], 1, col2);
+        for (int j = 0; j < col2; j++) {
+          rec.e[(size_t)r * kRow + j] = (-(S)dibp) * wbp[1 + j];
+          rec.v[(size_t)r * kRow + j] = v[1 + j];
         }
       }
     }
     if (!grid_barrier(&ws->bar, target)) return fail();
-    const int cnt = *(volatile int*)&ws->cnt;
+    if (lead) {
+      walk_records_in_order<R, H, S>(c, rec, cnt, sm);
+      if (threadIdx.x == 0) {
+        ws->done = sm.done;
+        ws->last_hi = __ldcg(&rec.hi[cnt - 1]);
+        ws->last_lo = __ldcg(&rec.lo[cnt - 1]);
+      }
+    }
+    if (!grid_barrier(&ws->bar, target)) return fail();
     const int done = *(volatile int*)&ws->done;
     consumed += cnt;
-    if (done || consumed >= L || cnt == 0) break;
+    if (done || consumed >= L) break;
     last = Key96{*(volatile unsigned long long*)&ws->last_hi, *(volatile unsigned int*)&ws->last_lo};
     first_round = false;
+    want = 2 * want < walk_rows(c.n) ? 2 * want : walk_rows(c.n);
   }
-  if (!lead || threadIdx.x != 0) return;
-  if (sm.done == 2) return;  // a failed M*wbp: the driver resets the memory
-  walk_end(st, w, sm.work[0]);
+  // the walk's end into the state (walk_end), M c by the first warp
+  if (!lead || threadIdx.x >= 32) return;
+  if (!sm.all_fixed) {
+    if (lane == 0) {
+      if (sm.dtm <= S(0)) sm.dtm = 0;
+      sm.tsum = sm.tsum + sm.dtm;
+    }
+    __syncwarp();
+    if (lane < col2) st->c[lane + 1] += sm.dtm * st->p[lane + 1];
+  }
+  if (lane == 0) {
+    st->f1 = sm.f1;
+    st->f2 = sm.f2;
+    st->dtm = sm.dtm;
+    st->tsum = sm.tsum;
+    st->tj = sm.tj;
+    st->nleft = sm.nleft;
+    st->nint = sm.nint;
+  }
+  if (lane < col2) sm.wbp[0][lane + 1] = st->c[lane + 1];
+  __syncwarp();
+  if (col > 0) {
+    const int info = wbmv(sm.sy, sm.wt, col, sm.wbp[0], sm.bv[0], sm.work[0], lane);
+    if (info != 0) {
+      if (lane == 0) st->internal_fail = -8;
+      return;
+    }
+    if (lane < col2) st->mc[lane + 1] = sm.bv[0][lane + 1];
+  }
+  if (lane == 0) st->gcp_state = GCP_DONE;
 }
 
 }  // namespace lbfgsb_b200
