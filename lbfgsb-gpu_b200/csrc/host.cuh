@@ -296,7 +296,7 @@ struct Plan {
 };
 
 // Takes one solve's workspace from the pool, checks its alignment, fills the pass context
-// and the launch shapes, zeroes the history, and fills the host copy of the state (w.hs)
+// and the launch shapes, and fills the host copy of the state (w.hs)
 // with the start of the reference driver (head = 1, theta = 1, col = 0).  walk: allocate
 // the breakpoint-walk buffers now (device-driven solves cannot allocate them on demand).
 template <typename R, typename H, typename S>
@@ -392,9 +392,9 @@ static void prepare(Workspace<R, H, S>& w, Ctx<R, H, S>& c, Plan& p, int n, int 
   c.part = w.part;
   p.g_elem = (int)std::min<long long>(((long long)n + 255) / 256, (long long)device_sms() * 8);
 
-  // history slots start at zero so that unused positions read as finite values
-  CK(cudaMemsetAsync(w.ws, 0, N * kSlots * sizeof(H), stream));
-  CK(cudaMemsetAsync(w.wy, 0, N * kSlots * sizeof(H), stream));
+  // the history needs no clearing: every pass reads the col live slots only, which a
+  // post-evaluation pass has written (clearing it took 2 x 193 us of a 23 ms solve of 12
+  // iterations at n = 4096^2 FP64)
   CK(cudaMemsetAsync(w.fbits, 0, words * sizeof(uint32_t), stream));
   CK(cudaMemsetAsync(w.ticket, 0, sizeof(unsigned int), stream));
 
