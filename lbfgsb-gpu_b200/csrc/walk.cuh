@@ -483,10 +483,12 @@ __device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned int& ta
 //   scan    p += (-dibp) wbp and c += dt p need no f' or f'': one lane per component, one
 //           dependent addition a key;
 //   dots    wbp'M c and wbp'M p, one thread per key, and the terms of f' and f'';
-//   chain   f' and f'': three or four dependent additions each a key, on one thread (the
-//           walk's rate: the reference's order of these additions is kept); sum of dt beside;
+//   f''     three dependent additions a key on one thread;
+//   f'      four dependent additions a key on one thread (the walk's rate: the reference's
+//           order of these additions is kept), and the sum of dt on another;
 //   test    dtm = -f'/f'' against the next breakpoint's distance, one lane per key.
-// The keys after the one where the walk ends are worked on in vain (at most four sub-batches).
+// The keys after the one where the walk ends are worked on in vain (at most five sub-batches).
+// f' and f'' on one thread, their terms loaded four keys at a time, took 38-45 ns a key.
 //
 // One thread walking key by key, with 64 rows of M*wbp prepared at a time by 64 threads,
 // took 0.46-0.52 us a breakpoint (n = 512^2, 217,112 breakpoints in one walk: 112 ms).
@@ -537,61 +539,79 @@ struct WalkCoop {
   unsigned int k_lo[kPiece];
   unsigned int hist[256];
   S sy[kMaxM * kMaxM], wt[kMaxM * kMaxM];
+  int slot[kMaxM];  // the ring's physical slots, oldest pair first
+  int rank[kBatch];
   S wbp[kBatch][kRow + 1], bv[kBatch][kRow + 1], work[kBatch][kMaxM + 1];
-  // CTA 0's pipeline; buffers are indexed by sub-batch modulo their count
-  S e[2][kSub][kRow];
-  S p[2][kSub][kRow + 1], c[2][kSub][kRow + 1];  // p before, c after each key
-  S dt[8][kSub];
-  S a1[2][kSub], a2[2][kSub], a3[2][kSub], b1[2][kSub], b2[2][kSub], b3[2][kSub];
-  S f1s[2][kSub], f2s[2][kSub], ts[2][kSub];     // after each key
-  S ckp[kWalkRows / kSub][kRow], ckc[kWalkRows / kSub][kRow];  // p, c before each sub-batch
+  union {
+    struct {
+      // CTA 0's pipeline; buffers are indexed by sub-batch modulo their count
+      S e[2][kSub][kRow];
+      S p[2][kSub][kRow + 1], c[2][kSub][kRow + 1];  // p before, c after each key
+      S dt[8][kSub];
+      S a[4][kSub][4];                               // the terms of f' (the first becomes dt f'')
+      S b[2][kSub][4];                               // the terms of f''
+      S f1s[2][kSub], f2s[4][kSub], ts[2][kSub];     // after each key
+      S ckp[kWalkRows / kSub][kRow], ckc[kWalkRows / kSub][kRow];  // p, c before each sub-batch
+    };
+    struct {  // every CTA: the chunk's keys while they are ranked
+      unsigned long long all_hi[kWalkRows];
+      unsigned int all_lo[kWalkRows];
+    };
+  };
   S f1, f2, dtm, tsum, tj;                       // before the next key to be tested
   int nleft, nint, all_fixed, done, stop, passed, info;
 };
 
-// Sorts the kPiece keys of sm.k_hi / k_lo (all threads of the CTA, one key each).
+// Sorts the kPiece keys held one per thread (a bitonic network; partners within a warp by
+// shuffles, farther ones through shared memory).
 template <typename S>
-__device__ void sort_piece(WalkCoop<S>& sm) {
+__device__ Key96 sort_piece(WalkCoop<S>& sm, Key96 k) {
   const int e = (int)threadIdx.x;
+#pragma unroll 1
   for (int size = 2; size <= kPiece; size <<= 1) {
+#pragma unroll 1
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      __syncthreads();
-      const int p = e ^ stride;
-      if (p > e) {
-        const bool up = (e & size) == 0;
-        const Key96 a{sm.k_hi[e], sm.k_lo[e]}, b{sm.k_hi[p], sm.k_lo[p]};
-        if (key_less(b, a) == up) {
-          sm.k_hi[e] = b.hi;
-          sm.k_lo[e] = b.lo;
-          sm.k_hi[p] = a.hi;
-          sm.k_lo[p] = a.lo;
-        }
+      Key96 o;
+      if (stride >= 32) {
+        sm.k_hi[e] = k.hi;
+        sm.k_lo[e] = k.lo;
+        __syncthreads();
+        o = Key96{sm.k_hi[e ^ stride], sm.k_lo[e ^ stride]};
+        __syncthreads();
+      } else {
+        o.hi = __shfl_xor_sync(0xffffffffu, k.hi, stride);
+        o.lo = __shfl_xor_sync(0xffffffffu, k.lo, stride);
       }
+      // the lower of the pair keeps the smaller key where the run ascends
+      const bool want_small = ((e & stride) == 0) == ((e & size) == 0);
+      if (key_less(o, k) == want_small) k = o;
     }
   }
-  __syncthreads();
+  return k;
 }
 
-// Rank of key k (position q of the pieces, each sorted) among the chunk's cnt keys.
-template <typename S>
-__device__ __forceinline__ int chunk_rank(const WalkRecords<S>& rec, const Key96& k, int q, int cnt) {
-  int lb[kMaxPieces];
+// The pieces (each sorted, in shared memory) below key k of piece `own`: the lower bounds of k in
+// the pieces first, first + kRankLanes, ... of the chunk's cnt keys.
+constexpr int kRankLanes = 4;  // threads that share a key's pieces
+__device__ __forceinline__ int rank_part(const unsigned long long* all_hi, const unsigned int* all_lo,
+                                         const Key96& k, int own, int first, int cnt) {
+  constexpr int kMine = kMaxPieces / kRankLanes;
+  int lb[kMine];
 #pragma unroll
-  for (int pc = 0; pc < kMaxPieces; pc++) lb[pc] = 0;
-  const int own = q / kPiece;
+  for (int u = 0; u < kMine; u++) lb[u] = 0;
+#pragma unroll 1
   for (int step = kPiece; step > 0; step >>= 1) {
 #pragma unroll
-    for (int pc = 0; pc < kMaxPieces; pc++) {
-      const int base = pc * kPiece, at = lb[pc] + step;
-      if (pc != own && at <= kPiece && base + at <= cnt) {
-        const Key96 o{__ldcg(&rec.raw_hi[base + at - 1]), __ldcg(&rec.raw_lo[base + at - 1])};
-        if (key_less(o, k)) lb[pc] = at;
-      }
+    for (int u = 0; u < kMine; u++) {
+      const int pc = first + u * kRankLanes, base = pc * kPiece, at = lb[u] + step;
+      if (pc != own && at <= kPiece && base + at <= cnt &&
+          key_less(Key96{all_hi[base + at - 1], all_lo[base + at - 1]}, k))
+        lb[u] = at;
     }
   }
-  int r = q - own * kPiece;
+  int r = 0;
 #pragma unroll
-  for (int pc = 0; pc < kMaxPieces; pc++) r += lb[pc];
+  for (int u = 0; u < kMine; u++) r += lb[u];
   return r;
 }
 
@@ -609,6 +629,83 @@ __device__ __forceinline__ S row_dot(const S* b, const S (&a)[kRow], int col2) {
     }
   }
   return r;
+}
+
+// f'' after each of nk keys: f2 - b[0] + b[1] - b[2] (lbfgsbcpu.cpp:789, 800-803; the last two
+// terms with a history only), no lower than floor2 when kLimit.  One thread; the terms of the
+// next keys are loaded while these are added.
+constexpr int kWalkGroup = 4;
+template <bool kHist, bool kLimit, typename S>
+__device__ __forceinline__ void walk_f2(const S (*b)[4], S* out, int nk, S f2, S floor2) {
+  constexpr int U = kWalkGroup, T = kHist ? 3 : 1;
+  S t[U][T];
+  auto load = [&](int q) {
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+      for (int w = 0; w < T; w++) t[u][w] = b[q + u][w];
+  };
+  auto step = [&](const S* v) {
+    f2 = f2 - v[0];
+    if constexpr (kHist) f2 = f2 + v[1] - v[2];
+    if constexpr (kLimit) f2 = smax(floor2, f2);
+  };
+  int q = 0;
+  if (nk >= U) load(0);
+  for (; q + U <= nk; q += U) {
+    S v[U][T];
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+      for (int w = 0; w < T; w++) v[u][w] = t[u][w];
+    if (q + 2 * U <= nk) load(q + U);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      step(v[u]);
+      out[q + u] = f2;
+    }
+  }
+  for (; q < nk; q++) {
+    step(b[q]);
+    out[q] = f2;
+  }
+}
+
+// f' after each of nk keys: f1 + a[0] + a[1] - a[2] + a[3] (788, 801; the last with a history
+// only), as walk_f2.
+template <bool kHist, typename S>
+__device__ __forceinline__ void walk_f1(const S (*a)[4], S* out, int nk, S f1) {
+  constexpr int U = kWalkGroup;
+  S t[U][4];
+  auto load = [&](int q) {
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+      for (int w = 0; w < (kHist ? 4 : 3); w++) t[u][w] = a[q + u][w];
+  };
+  int q = 0;
+  if (nk >= U) load(0);
+  for (; q + U <= nk; q += U) {
+    S v[U][4];
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+      for (int w = 0; w < (kHist ? 4 : 3); w++) v[u][w] = t[u][w];
+    if (q + 2 * U <= nk) load(q + U);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      f1 = f1 + v[u][0] + v[u][1] - v[u][2];
+      if (kHist) f1 = f1 + v[u][3];
+      v[u][0] = f1;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) out[q + u] = v[u][0];
+  }
+  for (; q < nk; q++) {
+    f1 = f1 + a[q][0] + a[q][1] - a[q][2];
+    if (kHist) f1 = f1 + a[q][3];
+    out[q] = f1;
+  }
 }
 
 // CTA 0: walks the cnt records in order (all threads).  sm.f1 .. sm.nint carry the walk from
@@ -643,10 +740,21 @@ __device__ void walk_records_in_order(const Ctx<R, H, S>& c, const WalkRecords<S
   }
   stage(0, threadIdx.x, blockDim.x);
   __syncthreads();
-  for (int s = 0; s < nsub + 3; s++) {
+  for (int s = 0; s < nsub + 4; s++) {
     if (warp >= 8) {
       if (s + 1 < nsub) stage(s + 1, (int)threadIdx.x - 256, (int)blockDim.x - 256);
     } else if (warp == 0) {
+      if (lane == kRow && s >= 3 && s - 3 < nsub) {
+        // the sum of dt, at the pace of f'
+        const int b = s - 3, nk = cnt - b * kSub < kSub ? cnt - b * kSub : kSub;
+        const S* dt = sm.dt[b & 7];
+        S ts = b > 0 ? sm.ts[(b - 1) & 1][kSub - 1] : sm.tsum;
+#pragma unroll 8
+        for (int q = 0; q < nk; q++) {
+          ts = ts + dt[q];
+          sm.ts[b & 1][q] = ts;
+        }
+      }
       if (s < nsub && col2 > 0 && lane < kRow) {
         const int b = s & 1, nk = cnt - s * kSub < kSub ? cnt - s * kSub : kSub;
         const S* dt = sm.dt[s & 7];
@@ -678,117 +786,76 @@ __device__ void walk_records_in_order(const Ctx<R, H, S>& c, const WalkRecords<S
     } else if (warp >= 4) {
       const int b = s - 1, q = (int)threadIdx.x - 128;
       if (b >= 0 && b < nsub && b * kSub + q < cnt) {
-        const int k = b * kSub + q, o = b & 1;
+        const int k = b * kSub + q, o = b & 1, oa = b & 3;
         const S dibp = __ldcg(&rec.dibp[k]), zibp = __ldcg(&rec.zibp[k]);
         const S dibp2 = dibp * dibp;
-        sm.a1[o][q] = dibp2;
-        sm.a2[o][q] = theta * dibp * zibp;
-        sm.b1[o][q] = theta * dibp2;
+        sm.a[oa][q][1] = dibp2;
+        sm.a[oa][q][2] = theta * dibp * zibp;
+        sm.b[o][q][0] = theta * dibp2;
         if (col2 > 0) {
           S v[kRow];
 #pragma unroll
           for (int j = 0; j < kRow; j++) v[j] = j < col2 ? __ldcg(&rec.v[(size_t)k * kRow + j]) : S(0);
           const S wmw = __ldcg(&rec.wmw[k]);
           const S wmc = row_dot(sm.c[o][q], v, col2), wmp = row_dot(sm.p[o][q], v, col2);
-          sm.a3[o][q] = dibp * wmc;
-          sm.b2[o][q] = (S)2.0 * dibp * wmp;
-          sm.b3[o][q] = dibp2 * wmw;
+          sm.a[oa][q][3] = dibp * wmc;
+          sm.b[o][q][1] = (S)2.0 * dibp * wmp;
+          sm.b[o][q][2] = dibp2 * wmw;
         }
       }
     } else if (warp == 1) {
       const int b = s - 2;
-      if (lane == 0 && b >= 0 && b < nsub) {
-        const int o = b & 1, nk = cnt - b * kSub < kSub ? cnt - b * kSub : kSub;
-        const S* dt = sm.dt[b & 7];
-        // f' and f'' after the last key of the sub-batch before
-        S f1 = b > 0 ? sm.f1s[o ^ 1][kSub - 1] : sm.f1, f2 = b > 0 ? sm.f2s[o ^ 1][kSub - 1] : sm.f2;
-        constexpr int U = 4;
-        int q = 0;
-        for (; q + U <= nk; q += U) {
-          S d[U], a1[U], a2[U], a3[U], b1[U], b2[U], b3[U];
-#pragma unroll
-          for (int u = 0; u < U; u++) {
-            d[u] = dt[q + u];
-            a1[u] = sm.a1[o][q + u];
-            a2[u] = sm.a2[o][q + u];
-            b1[u] = sm.b1[o][q + u];
-            a3[u] = sm.a3[o][q + u];
-            b2[u] = sm.b2[o][q + u];
-            b3[u] = sm.b3[o][q + u];
-          }
-          // without the lower limit of f'', which hardly ever acts; if it does, once more
-          const S g1 = f1, g2 = f2;
-          bool low = false;
-          S r1[U], r2[U];
-#pragma unroll
-          for (int u = 0; u < U; u++) {
-            f1 = f1 + d[u] * f2 + a1[u] - a2[u];
-            f2 = f2 - b1[u];
-            if (col2 > 0) {
-              f1 = f1 + a3[u];
-              f2 = f2 + b2[u] - b3[u];
-            }
-            low = low || floor2 > f2;
-            r1[u] = f1;
-            r2[u] = f2;
-          }
-          if (low) {
-            f1 = g1;
-            f2 = g2;
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-              f1 = f1 + d[u] * f2 + a1[u] - a2[u];
-              f2 = f2 - b1[u];
-              if (col2 > 0) {
-                f1 = f1 + a3[u];
-                f2 = f2 + b2[u] - b3[u];
-              }
-              f2 = smax(floor2, f2);
-              r1[u] = f1;
-              r2[u] = f2;
-            }
-          }
-#pragma unroll
-          for (int u = 0; u < U; u++) {
-            sm.f1s[o][q + u] = r1[u];
-            sm.f2s[o][q + u] = r2[u];
-          }
+      if (b >= 0 && b < nsub) {
+        const int nk = cnt - b * kSub < kSub ? cnt - b * kSub : kSub;
+        S* f2s = sm.f2s[b & 3];
+        const S f2 = b > 0 ? sm.f2s[(b - 1) & 3][kSub - 1] : sm.f2;
+        if (lane == 0) {
+          if (col2 > 0)
+            walk_f2<true, false>(sm.b[b & 1], f2s, nk, f2, floor2);
+          else
+            walk_f2<false, false>(sm.b[b & 1], f2s, nk, f2, floor2);
         }
-        for (; q < nk; q++) {
-          f1 = f1 + dt[q] * f2 + sm.a1[o][q] - sm.a2[o][q];
-          f2 = f2 - sm.b1[o][q];
-          if (col2 > 0) {
-            f1 = f1 + sm.a3[o][q];
-            f2 = f2 + sm.b2[o][q] - sm.b3[o][q];
-          }
-          f2 = smax(floor2, f2);
-          sm.f1s[o][q] = f1;
-          sm.f2s[o][q] = f2;
+        __syncwarp();
+        // the lower limit of f'' hardly ever acts: the sub-batch is summed without it, and
+        // once more with it when it would have acted
+        bool low = false;
+        for (int q = lane; q < nk; q += 32) low = low || floor2 > f2s[q];
+        if (__any_sync(0xffffffffu, low) && lane == 0) {
+          if (col2 > 0)
+            walk_f2<true, true>(sm.b[b & 1], f2s, nk, f2, floor2);
+          else
+            walk_f2<false, true>(sm.b[b & 1], f2s, nk, f2, floor2);
         }
       }
     } else if (warp == 2) {
-      const int b = s - 2;
-      if (lane == 0 && b >= 0 && b < nsub) {
-        const int o = b & 1, nk = cnt - b * kSub < kSub ? cnt - b * kSub : kSub;
+      const int b = s - 3;
+      if (b >= 0 && b < nsub) {
+        const int nk = cnt - b * kSub < kSub ? cnt - b * kSub : kSub;
         const S* dt = sm.dt[b & 7];
-        S ts = b > 0 ? sm.ts[o ^ 1][kSub - 1] : sm.tsum;
-#pragma unroll 4
-        for (int q = 0; q < nk; q++) {
-          ts = ts + dt[q];
-          sm.ts[o][q] = ts;
+        const S* f2s = sm.f2s[b & 3];
+        const S f2 = b > 0 ? sm.f2s[(b - 1) & 3][kSub - 1] : sm.f2;  // before the sub-batch
+        for (int q = lane; q < nk; q += 32) sm.a[b & 3][q][0] = dt[q] * (q > 0 ? f2s[q - 1] : f2);
+        __syncwarp();
+        if (lane == 0) {
+          const S f1 = b > 0 ? sm.f1s[(b - 1) & 1][kSub - 1] : sm.f1;
+          if (col2 > 0)
+            walk_f1<true>(sm.a[b & 3], sm.f1s[b & 1], nk, f1);
+          else
+            walk_f1<false>(sm.a[b & 3], sm.f1s[b & 1], nk, f1);
         }
       }
     } else {  // warp 3
-      const int b = s - 3;
+      const int b = s - 4;
       if (b >= 0) {
         const int o = b & 1, base = b * kSub, nk = cnt - base < kSub ? cnt - base : kSub;
         const S* dt = sm.dt[b & 7];
+        const S* f2s = sm.f2s[b & 3];
         int hit = -1;
         for (int r = 0; r < nk && hit < 0; r += 32) {
           const int q = r + lane;
           bool ends = false;
           if (q < nk) {
-            const S dtm = q == 0 ? sm.dtm : -sm.f1s[o][q - 1] / sm.f2s[o][q - 1];
+            const S dtm = q == 0 ? sm.dtm : -sm.f1s[o][q - 1] / f2s[q - 1];
             ends = dtm < dt[q];
           }
           const unsigned bal = __ballot_sync(0xffffffffu, ends);
@@ -805,7 +872,7 @@ __device__ void walk_records_in_order(const Ctx<R, H, S>& c, const WalkRecords<S
           if (q > 0) sm.tsum = sm.ts[o][q - 1];
           if (f > 0) {
             sm.f1 = sm.f1s[o][f - 1];
-            sm.f2 = sm.f2s[o][f - 1];
+            sm.f2 = f2s[f - 1];
             sm.dtm = -sm.f1 / sm.f2;
           }
           if (fixed) {
@@ -855,7 +922,7 @@ __device__ void walk_records_in_order(const Ctx<R, H, S>& c, const WalkRecords<S
 // Lists the breakpoints with the whole grid and walks them chunk by chunk.  wsc->bar and
 // *wl_n are zero at launch.
 template <typename R, typename H, typename S>
-__global__ void __launch_bounds__(kWalkThreads) k_walk_coop(Ctx<R, H, S> c, const R* __restrict__ x,
+__global__ void __launch_bounds__(kWalkThreads, 1) k_walk_coop(Ctx<R, H, S> c, const R* __restrict__ x,
                                                             const R* __restrict__ g) {
   DevState<S>* st = c.st;
   if (c.rounds) {
@@ -876,6 +943,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_coop(Ctx<R, H, S> c, cons
   if (threadIdx.x == 0) {
     // a zero on the factor's diagonal fails every M*wbp (the driver resets the memory)
     sm.info = 0;
+    for (int j = 0; j < col; j++) sm.slot[j] = st->phys[(st->head - 1 + j) % st->m + 1];
     for (int j = col; j >= 1; j--)
       if (LB_AT(st->wt, kMaxM, j, j) == S(0)) sm.info = j;
   }
@@ -914,9 +982,6 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_coop(Ctx<R, H, S> c, cons
   gather_breakpoints<R, H, S>(c, cta_here(), blockDim.x, x, g);
   if (!grid_barrier(&ws->bar, target)) return fail();
   const long long L = (long long)*(volatile unsigned int*)c.wl_n;
-  const H *Y[kMaxM], *Sl[kMaxM];
-  ring_ptrs(st, c.wy, c.ld, Y);
-  ring_ptrs(st, c.ws, c.ld, Sl);
   const long long stride = (long long)gridDim.x * blockDim.x;
   const long long e0 = (long long)blockIdx.x * blockDim.x;
   const int lane = threadIdx.x & 31;
@@ -994,48 +1059,68 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_coop(Ctx<R, H, S> c, cons
     // sort the pieces
     for (int pc = blockIdx.x; pc * kPiece < cnt; pc += gridDim.x) {
       const int q = pc * kPiece + (int)threadIdx.x;
-      sm.k_hi[threadIdx.x] = q < cnt ? __ldcg(&rec.raw_hi[q]) : ~0ull;
-      sm.k_lo[threadIdx.x] = q < cnt ? __ldcg(&rec.raw_lo[q]) : ~0u;
-      sort_piece(sm);
+      Key96 k{~0ull, ~0u};
+      if (q < cnt) k = Key96{__ldcg(&rec.raw_hi[q]), __ldcg(&rec.raw_lo[q])};
+      k = sort_piece(sm, k);
       if (q < cnt) {
-        rec.raw_hi[q] = sm.k_hi[threadIdx.x];
-        rec.raw_lo[q] = sm.k_lo[threadIdx.x];
+        rec.raw_hi[q] = k.hi;
+        rec.raw_lo[q] = k.lo;
       }
-      __syncthreads();
     }
     if (!grid_barrier(&ws->bar, target)) return fail();
     if (lead && threadIdx.x == 0) ws->chunk_n = 0;
-    // rank every key and prepare its record there, the keys spread over the CTAs
+    // rank every key and prepare its record there, the keys spread over the CTAs; every CTA
+    // searches a copy of the pieces in its shared memory (searching them in L2, all CTAs
+    // probing the same lines, took 34 us a chunk)
+#pragma unroll 4
+    for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
+      sm.all_hi[q] = __ldcg(&rec.raw_hi[q]);
+      sm.all_lo[q] = __ldcg(&rec.raw_lo[q]);
+    }
+    __syncthreads();
     for (int q0 = 0; q0 < cnt; q0 += kBatch * (int)gridDim.x) {
-      const int q = q0 + (int)threadIdx.x * (int)gridDim.x + (int)blockIdx.x;
-      if (threadIdx.x >= kBatch || q >= cnt) continue;
-      const Key96 k{__ldcg(&rec.raw_hi[q]), __ldcg(&rec.raw_lo[q])};
-      const int i = (int)k.lo;
-      S* wbp = sm.wbp[threadIdx.x];
-      S* v = sm.bv[threadIdx.x];
-      const R xi = x[i], gi = g[i];
+      if (threadIdx.x < kBatch * kRankLanes) {
+        const int qr = q0 + (int)(threadIdx.x / kRankLanes) * (int)gridDim.x + (int)blockIdx.x;
+        int r = 0;
+        if (qr < cnt)
+          r = rank_part(sm.all_hi, sm.all_lo, Key96{sm.all_hi[qr], sm.all_lo[qr]}, qr / kPiece,
+                        (int)(threadIdx.x % kRankLanes), cnt);
 #pragma unroll
-      for (int j = 0; j < kMaxM; j++)
-        if (j < col) {
-          wbp[1 + j] = (S)HistTraits<H>::load(Y[j] + i);
-          wbp[1 + col + j] = theta * (S)HistTraits<H>::load(Sl[j] + i);
+        for (int o = 1; o < kRankLanes; o <<= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+        if (threadIdx.x % kRankLanes == 0) sm.rank[threadIdx.x / kRankLanes] = r + qr % kPiece;
+      }
+      __syncthreads();
+      const int q = q0 + (int)threadIdx.x * (int)gridDim.x + (int)blockIdx.x;
+      if (threadIdx.x < kBatch && q < cnt) {
+        const Key96 k{sm.all_hi[q], sm.all_lo[q]};
+        const int i = (int)k.lo;
+        S* wbp = sm.wbp[threadIdx.x];
+        S* v = sm.bv[threadIdx.x];
+        const R xi = x[i], gi = g[i];
+#pragma unroll 4
+        for (int j = 0; j < col; j++) {
+          const size_t at = (size_t)sm.slot[j] * (size_t)c.ld + i;
+          wbp[1 + j] = (S)HistTraits<H>::load(c.wy + at);
+          wbp[1 + col + j] = theta * (S)HistTraits<H>::load(c.ws + at);
         }
-      const int r = chunk_rank(rec, k, q, cnt);
-      const R dibp = -gi;
-      const R zibp = (dibp > R(0)) ? rsub(c.u[i], xi) : rsub(c.l[i], xi);
-      rec.hi[r] = k.hi;
-      rec.lo[r] = k.lo;
-      rec.dibp[r] = (S)dibp;
-      rec.zibp[r] = (S)zibp;
-      if (col > 0) {
-        int info = 0;
-        sbmv(sm.sy, sm.wt, col, wbp, v, &info, sm.work[threadIdx.x]);
-        rec.wmw[r] = sdot(&wbp[1], 1, &v[1], 1, col2);
-        for (int j = 0; j < col2; j++) {
-          rec.e[(size_t)r * kRow + j] = (-(S)dibp) * wbp[1 + j];
-          rec.v[(size_t)r * kRow + j] = v[1 + j];
+        const int r = sm.rank[threadIdx.x];
+        const R dibp = -gi;
+        const R zibp = (dibp > R(0)) ? rsub(c.u[i], xi) : rsub(c.l[i], xi);
+        rec.hi[r] = k.hi;
+        rec.lo[r] = k.lo;
+        rec.dibp[r] = (S)dibp;
+        rec.zibp[r] = (S)zibp;
+        if (col > 0) {
+          int info = 0;
+          sbmv(sm.sy, sm.wt, col, wbp, v, &info, sm.work[threadIdx.x]);
+          rec.wmw[r] = sdot(&wbp[1], 1, &v[1], 1, col2);
+          for (int j = 0; j < col2; j++) {
+            rec.e[(size_t)r * kRow + j] = (-(S)dibp) * wbp[1 + j];
+            rec.v[(size_t)r * kRow + j] = v[1 + j];
+          }
         }
       }
+      __syncthreads();  // the ranks are rewritten
     }
     if (!grid_barrier(&ws->bar, target)) return fail();
     if (lead) {
