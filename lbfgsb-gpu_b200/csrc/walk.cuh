@@ -488,10 +488,12 @@ __device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned int& ta
 //           order of these additions is kept), and the sum of dt on another;
 //   test    dtm = -f'/f'' against the next breakpoint's distance, one lane per key.
 // The keys after the one where the walk ends are worked on in vain (at most five sub-batches).
-// f' and f'' on one thread, their terms loaded four keys at a time, took 38-45 ns a key.
 //
-// One thread walking key by key, with 64 rows of M*wbp prepared at a time by 64 threads,
-// took 0.46-0.52 us a breakpoint (n = 512^2, 217,112 breakpoints in one walk: 112 ms).
+// What bounds it: f', four dependent additions of 8.3 cycles each, 33-40 cycles a key; with the
+// chunk's selection, sort and preparation (40-60 us for 8192 keys) a key takes 35 ns.  One
+// thread walking key by key, with 64 rows of M*wbp prepared at a time by 64 threads, took
+// 0.46-0.52 us a key (n = 512^2, a solve with 426,000 keys in six walks: 190.7 -> 15.1 ms); f'
+// and f'' on one thread, and f' with its loads waited for, took 74-84 cycles a key (23.2 ms).
 constexpr int kWalkRows = 8192;       // breakpoints of a chunk at most
 constexpr int kWalkFirst = 1024;      // of the first chunk (most walks are short); then doubled
 constexpr int kPiece = kWalkThreads;  // keys sorted together
@@ -548,9 +550,9 @@ struct WalkCoop {
       S e[2][kSub][kRow];
       S p[2][kSub][kRow + 1], c[2][kSub][kRow + 1];  // p before, c after each key
       S dt[8][kSub];
-      S a[4][kSub][4];                               // the terms of f' (the first becomes dt f'')
-      S b[2][kSub][4];                               // the terms of f''
-      S f1s[2][kSub], f2s[4][kSub], ts[2][kSub];     // after each key
+      alignas(16) S a[4][kSub][4];                               // the terms of f' (the first becomes dt f'')
+      alignas(16) S b[2][kSub][4];                               // the terms of f''
+      alignas(16) S f1s[2][kSub], f2s[4][kSub], ts[2][kSub];     // after each key
       S ckp[kWalkRows / kSub][kRow], ckc[kWalkRows / kSub][kRow];  // p, c before each sub-batch
     };
     struct {  // every CTA: the chunk's keys while they are ranked
@@ -631,81 +633,77 @@ __device__ __forceinline__ S row_dot(const S* b, const S (&a)[kRow], int col2) {
   return r;
 }
 
+// Four values in one (float) or two (double) shared-memory loads, and back.
+__device__ __forceinline__ void lds4(uint32_t at, double (&v)[4]) {
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "r"(at) : "memory");
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v[2]), "=d"(v[3]) : "r"(at + 16) : "memory");
+}
+__device__ __forceinline__ void lds4(uint32_t at, float (&v)[4]) {
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void sts4(uint32_t at, const double (&v)[4]) {
+  asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(at), "d"(v[0]), "d"(v[1]) : "memory");
+  asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(at + 16), "d"(v[2]), "d"(v[3]) : "memory");
+}
+__device__ __forceinline__ void sts4(uint32_t at, const float (&v)[4]) {
+  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3])
+               : "memory");
+}
+
+// One thread runs a chain over nk keys, a row of four terms each: step(row) returns the chain's
+// value after the key, stored to out.  Groups of four keys, the next group's rows loaded while
+// one group is added (two register sets, so that no addition waits for a load).
+template <typename S, typename Step>
+__device__ __forceinline__ void walk_chain(const S (*rows)[4], S* out, int nk, Step&& step) {
+  constexpr int U = 4;
+  const uint32_t in = smem_addr(rows), o = smem_addr(out);
+  constexpr uint32_t kB = 4 * sizeof(S);
+  S va[U][4], vb[U][4];
+  auto load = [&](S (&v)[U][4], int q) {
+#pragma unroll
+    for (int u = 0; u < U; u++) lds4(in + (uint32_t)(q + u) * kB, v[u]);
+  };
+  auto run = [&](const S (&v)[U][4], int q) {
+    S r[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) r[u] = step(v[u]);
+    sts4(o + (uint32_t)q * (uint32_t)sizeof(S), r);
+  };
+  // (rows past nk, of a buffer of kSub, are loaded and not used)
+  int q = 0;
+  load(va, 0);
+#pragma unroll 1
+  for (; q + 2 * U <= nk; q += 2 * U) {
+    load(vb, q + U);
+    run(va, q);
+    load(va, q + 2 * U < kSub ? q + 2 * U : 0);
+    run(vb, q + U);
+  }
+  for (; q < nk; q++) out[q] = step(rows[q]);
+}
+
 // f'' after each of nk keys: f2 - b[0] + b[1] - b[2] (lbfgsbcpu.cpp:789, 800-803; the last two
-// terms with a history only), no lower than floor2 when kLimit.  One thread; the terms of the
-// next keys are loaded while these are added.
-constexpr int kWalkGroup = 4;
+// terms with a history only), no lower than floor2 when kLimit.
 template <bool kHist, bool kLimit, typename S>
 __device__ __forceinline__ void walk_f2(const S (*b)[4], S* out, int nk, S f2, S floor2) {
-  constexpr int U = kWalkGroup, T = kHist ? 3 : 1;
-  S t[U][T];
-  auto load = [&](int q) {
-#pragma unroll
-    for (int u = 0; u < U; u++)
-#pragma unroll
-      for (int w = 0; w < T; w++) t[u][w] = b[q + u][w];
-  };
-  auto step = [&](const S* v) {
+  walk_chain(b, out, nk, [&](const S* v) {
     f2 = f2 - v[0];
     if constexpr (kHist) f2 = f2 + v[1] - v[2];
     if constexpr (kLimit) f2 = smax(floor2, f2);
-  };
-  int q = 0;
-  if (nk >= U) load(0);
-  for (; q + U <= nk; q += U) {
-    S v[U][T];
-#pragma unroll
-    for (int u = 0; u < U; u++)
-#pragma unroll
-      for (int w = 0; w < T; w++) v[u][w] = t[u][w];
-    if (q + 2 * U <= nk) load(q + U);
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      step(v[u]);
-      out[q + u] = f2;
-    }
-  }
-  for (; q < nk; q++) {
-    step(b[q]);
-    out[q] = f2;
-  }
+    return f2;
+  });
 }
 
 // f' after each of nk keys: f1 + a[0] + a[1] - a[2] + a[3] (788, 801; the last with a history
-// only), as walk_f2.
+// only).
 template <bool kHist, typename S>
 __device__ __forceinline__ void walk_f1(const S (*a)[4], S* out, int nk, S f1) {
-  constexpr int U = kWalkGroup;
-  S t[U][4];
-  auto load = [&](int q) {
-#pragma unroll
-    for (int u = 0; u < U; u++)
-#pragma unroll
-      for (int w = 0; w < (kHist ? 4 : 3); w++) t[u][w] = a[q + u][w];
-  };
-  int q = 0;
-  if (nk >= U) load(0);
-  for (; q + U <= nk; q += U) {
-    S v[U][4];
-#pragma unroll
-    for (int u = 0; u < U; u++)
-#pragma unroll
-      for (int w = 0; w < (kHist ? 4 : 3); w++) v[u][w] = t[u][w];
-    if (q + 2 * U <= nk) load(q + U);
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      f1 = f1 + v[u][0] + v[u][1] - v[u][2];
-      if (kHist) f1 = f1 + v[u][3];
-      v[u][0] = f1;
-    }
-#pragma unroll
-    for (int u = 0; u < U; u++) out[q + u] = v[u][0];
-  }
-  for (; q < nk; q++) {
-    f1 = f1 + a[q][0] + a[q][1] - a[q][2];
-    if (kHist) f1 = f1 + a[q][3];
-    out[q] = f1;
-  }
+  walk_chain(a, out, nk, [&](const S* v) {
+    f1 = f1 + v[0] + v[1] - v[2];
+    if constexpr (kHist) f1 = f1 + v[3];
+    return f1;
+  });
 }
 
 // CTA 0: walks the cnt records in order (all threads).  sm.f1 .. sm.nint carry the walk from
@@ -719,15 +717,29 @@ __device__ void walk_records_in_order(const Ctx<R, H, S>& c, const WalkRecords<S
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nsub = (cnt + kSub - 1) / kSub;
   auto t_of = [&](int k) { return (S)__longlong_as_double((long long)__ldcg(&rec.hi[k])); };
-  auto stage = [&](int b, int tid, int nt) {
+  // sub-batch b into shared memory, by nt threads; every load is issued before the first store
+  auto stage = [&](int b, int tid, auto nt) {
+    constexpr int NT = decltype(nt)::value, kTrips = (kSub * kRow + NT - 1) / NT;
     const int base = b * kSub, nk = cnt - base < kSub ? cnt - base : kSub;
-    for (int q = tid; q < nk; q += nt) {
+    S v[kTrips];
+    if (col2 > 0) {
+#pragma unroll
+      for (int w = 0; w < kTrips; w++) {
+        const int q = tid + w * NT;
+        v[w] = q < nk * kRow ? __ldcg(&rec.e[(size_t)base * kRow + q]) : S(0);
+      }
+    }
+    for (int q = tid; q < nk; q += NT) {
       const int k = base + q;
       sm.dt[b & 7][q] = t_of(k) - (k > 0 ? t_of(k - 1) : sm.tj);
     }
-    if (col2 > 0)
-      for (int q = tid; q < nk * kRow; q += nt)
-        (&sm.e[b & 1][0][0])[q] = __ldcg(&rec.e[(size_t)base * kRow + q]);
+    if (col2 > 0) {
+#pragma unroll
+      for (int w = 0; w < kTrips; w++) {
+        const int q = tid + w * NT;
+        if (q < nk * kRow) (&sm.e[b & 1][0][0])[q] = v[w];
+      }
+    }
   };
   S pj = 0, cj = 0;  // warp 0: component `lane` of p and c
   if (warp == 0 && lane < col2) {
@@ -738,13 +750,11 @@ __device__ void walk_records_in_order(const Ctx<R, H, S>& c, const WalkRecords<S
     sm.stop = 0;
     sm.passed = cnt;
   }
-  stage(0, threadIdx.x, blockDim.x);
+  stage(0, (int)threadIdx.x, std::integral_constant<int, kWalkThreads>{});
   __syncthreads();
   for (int s = 0; s < nsub + 4; s++) {
-    if (warp >= 8) {
-      if (s + 1 < nsub) stage(s + 1, (int)threadIdx.x - 256, (int)blockDim.x - 256);
-    } else if (warp == 0) {
-      if (lane == kRow && s >= 3 && s - 3 < nsub) {
+    if (warp == kWalkThreads / 32 - 1) {
+      if (lane == 0 && s >= 3 && s - 3 < nsub) {
         // the sum of dt, at the pace of f'
         const int b = s - 3, nk = cnt - b * kSub < kSub ? cnt - b * kSub : kSub;
         const S* dt = sm.dt[b & 7];
@@ -755,26 +765,40 @@ __device__ void walk_records_in_order(const Ctx<R, H, S>& c, const WalkRecords<S
           sm.ts[b & 1][q] = ts;
         }
       }
+    } else if (warp >= 8) {
+      if (s + 1 < nsub) stage(s + 1, (int)threadIdx.x - 256, std::integral_constant<int, kWalkThreads - 256 - 32>{});
+    } else if (warp == 0) {
       if (s < nsub && col2 > 0 && lane < kRow) {
         const int b = s & 1, nk = cnt - s * kSub < kSub ? cnt - s * kSub : kSub;
         const S* dt = sm.dt[s & 7];
         sm.ckp[s][lane] = pj;
         sm.ckc[s][lane] = cj;
-        int q = 0;
-        for (; q + 8 <= nk; q += 8) {
-          S d[8], e[8];
+        constexpr int U = 4;
+        S da[U], ea[U], db[U], eb[U];
+        auto load = [&](S (&d)[U], S (&e)[U], int q) {
 #pragma unroll
-          for (int u = 0; u < 8; u++) {
+          for (int u = 0; u < U; u++) {
             d[u] = dt[q + u];
             e[u] = sm.e[b][q + u][lane];
           }
+        };
+        auto run = [&](const S (&d)[U], const S (&e)[U], int q) {
 #pragma unroll
-          for (int u = 0; u < 8; u++) {
+          for (int u = 0; u < U; u++) {
             sm.p[b][q + u][lane] = pj;
             cj += d[u] * pj;
             sm.c[b][q + u][lane] = cj;
             pj += e[u];
           }
+        };
+        int q = 0;
+        load(da, ea, 0);
+#pragma unroll 1
+        for (; q + 2 * U <= nk; q += 2 * U) {
+          load(db, eb, q + U);
+          run(da, ea, q);
+          load(da, ea, q + 2 * U < kSub ? q + 2 * U : 0);
+          run(db, eb, q + U);
         }
         for (; q < nk; q++) {
           sm.p[b][q][lane] = pj;
