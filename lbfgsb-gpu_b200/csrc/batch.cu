@@ -55,25 +55,25 @@ __device__ __forceinline__ int batch_instance(const int* first, int count, CtaPo
 }
 
 template <typename R, typename H, typename S, int CONS>
-__global__ void __launch_bounds__(CONS + 32) kb_gcp_scan(BatchLaunch<R, H, S> b) {
+__global__ void __launch_bounds__(cta_threads(CONS)) kb_gcp_scan(BatchLaunch<R, H, S> b) {
   CtaPos cp;
   const int k = batch_instance(b.first, b.count, cp);
   gcp_scan_pass<R, H, S, CONS>(b.table[k], cp, b.stages, nullptr, nullptr);
 }
 template <typename R, typename H, typename S, int CONS>
-__global__ void __launch_bounds__(CONS + 32) kb_freev_formk(BatchLaunch<R, H, S> b) {
+__global__ void __launch_bounds__(cta_threads(CONS)) kb_freev_formk(BatchLaunch<R, H, S> b) {
   CtaPos cp;
   const int k = batch_instance(b.first, b.count, cp);
   freev_formk_pass<R, H, S, CONS>(b.table[k], cp, b.stages, nullptr, nullptr);
 }
 template <typename R, typename H, typename S, int CONS>
-__global__ void __launch_bounds__(CONS + 32) kb_subsm_dir(BatchLaunch<R, H, S> b) {
+__global__ void __launch_bounds__(cta_threads(CONS)) kb_subsm_dir(BatchLaunch<R, H, S> b) {
   CtaPos cp;
   const int k = batch_instance(b.first, b.count, cp);
   subsm_dir_pass<R, H, S, CONS>(b.table[k], cp, b.stages, nullptr, nullptr, nullptr);
 }
 template <typename R, typename H, typename S, int CONS>
-__global__ void __launch_bounds__(CONS + 32) kb_subsm_apply(BatchLaunch<R, H, S> b) {
+__global__ void __launch_bounds__(cta_threads(CONS)) kb_subsm_apply(BatchLaunch<R, H, S> b) {
   CtaPos cp;
   const int k = batch_instance(b.first, b.count, cp);
   subsm_apply_pass<R, H, S, CONS>(b.table[k], cp, b.stages, nullptr, nullptr, nullptr);
@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(CONS + 32) kb_subsm_apply(BatchLaunch<R, H, S>
 // the post-evaluation pass with the next Cauchy scan for instances with bounds, the plain
 // one for the others (as the single-instance driver chooses)
 template <typename R, typename H, typename S, int CONS>
-__global__ void __launch_bounds__(CONS + 32) kb_post_gcp(BatchLaunch<R, H, S> b) {
+__global__ void __launch_bounds__(cta_threads(CONS)) kb_post_gcp(BatchLaunch<R, H, S> b) {
   CtaPos cp;
   const int k = batch_instance(b.first, b.count, cp);
   const Ctx<R, H, S>& c = b.table[k];
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(CONS + 32) kb_post_gcp(BatchLaunch<R, H, S> b)
   post_gcp_pass<R, H, S, CONS>(c, cp, b.stages, nullptr, nullptr, nullptr, nullptr, nullptr, S(0), 0);
 }
 template <typename R, typename H, typename S, int CONS>
-__global__ void __launch_bounds__(CONS + 32) kb_post_eval(BatchLaunch<R, H, S> b) {
+__global__ void __launch_bounds__(cta_threads(CONS)) kb_post_eval(BatchLaunch<R, H, S> b) {
   CtaPos cp;
   const int k = batch_instance(b.first, b.count, cp);
   const Ctx<R, H, S>& c = b.table[k];
@@ -641,7 +641,7 @@ class BatchRunner {
     const int rb = (cnt + 127) / 128;
     const BatchLaunch<R, H, S> bp{table_, first_pass_, cnt, 2};
     const BatchLaunch<R, H, S> be{table_, first_elem_, cnt, 2};
-    const int thr = kConsWide + 32;
+    const int thr = cta_threads(kConsWide);
     CK(cudaStreamBeginCapture(s_, cudaStreamCaptureModeThreadLocal));
     kb_round<R, H, S, RK_BEGIN><<<rb, 128, 0, s_>>>(table_, cnt);
     kb_gcp_scan<R, H, S, kConsWide><<<ctas_pass_, thr, ring_bytes(2, cap_gcp_), s_>>>(bp);

@@ -259,6 +259,70 @@ __device__ __forceinline__ S reduced_grad(bool uncon, R x, R z, R g, int col,
   return r;
 }
 
+// Scratch of a pass epilogue, one shared variable per kernel.
+template <typename S>
+struct EpiScratch {
+  SmallWork<S> sw;
+  S snap[4 * kMaxM * kMaxM];
+  double rp[20], rg[22];
+};
+template <typename S>
+__device__ __forceinline__ EpiScratch<S>& epi_scratch() {
+  __shared__ EpiScratch<S> x;
+  return x;
+}
+
+// The code of the two long epilogues (the free-set pass's and the fused post-evaluation pass's)
+// is fetched anew in each launch by the SM whose CTA ends last: about 40% of an epilogue's time
+// when the streaming part moves gigabytes in between.  So the epilogue is a function of its own
+// (__noinline__, one copy) called at two places: by the first warp of the last CTA, and, beside the
+// streaming, by the otherwise idle last warp of every CTA on the made-up state below, to no effect
+// but that the function's code is in the SM's instruction cache.  The made-up state takes the usual
+// path through every routine: a full ring that shifts, identity matrices, an accepted step.
+//
+// Below kWarmTiles tiles a CTA nothing is warmed: the last CTA would wait for its own warm-up, and
+// its code is still in L2 (n = 333^2, 1-2 tiles a CTA: 9% slower with the warm-up, n = 256^2 5%;
+// n = 1024^2 FP32, 13 tiles: 3% faster; 2048^2 mixed, 55 tiles: 3%).
+constexpr int kWarmTiles = 8;
+__device__ __forceinline__ bool worth_warming(int n, CtaPos cp) {
+  return n / kTile >= kWarmTiles * cp.count;
+}
+template <typename S>
+__device__ __forceinline__ void warm_state(int lane) {
+  unsigned int* words = reinterpret_cast<unsigned int*>(epi_state<S>());
+  for (int k = lane; k < (int)(sizeof(DevState<S>) / 4); k += 32) words[k] = 0;
+  __syncwarp();
+  DevState<S>* st = epi_state<S>();
+  if (lane < kMaxM) {
+    LB_AT(st->sy, kMaxM, lane + 1, lane + 1) = 1;
+    LB_AT(st->ss, kMaxM, lane + 1, lane + 1) = 1;
+    LB_AT(st->wt, kMaxM, lane + 1, lane + 1) = 1;
+  }
+  if (lane < 2 * kMaxM) {
+    LB_AT(st->wn, 2 * kMaxM, lane + 1, lane + 1) = 1;
+    LB_AT(st->wn1, 2 * kMaxM, lane + 1, lane + 1) = 1;
+  }
+  if (lane == 0) {
+    st->m = kMaxM;
+    st->cnstnd = 1;
+    st->col = 2;
+    st->head = 1;
+    st->itail = 2;
+    st->iupdat = kMaxM + 1;
+    st->updatd = 1;
+    st->theta = 1;
+    st->stp = 1;
+    st->stpmx = 2;
+    st->dtd = 1;
+    st->gdold = -1;
+    st->csave = 1;
+    st->ls.dsave[1] = -1;  // the initial slope
+    st->ls.dsave[5] = 1;   // the initial f: f = 0 converges
+    st->ls.dsave[11] = 2;
+  }
+  __syncwarp();
+}
+
 // cauchy's epilogue (lbfgsbcpu.cpp:702-733) and the first breakpoint test of the walk
 // (745-747), from the sums of the scan over the movable variables: red[0] sum g^2,
 // red[1..8] / red[9..16] the y / s parts of p = W'd by ring position, red[17] nbreak,
@@ -274,15 +338,12 @@ __device__ void gcp_epilogue(DevState<S>* st, const double* red, int col, SmallW
   const S f1 = -(S)red[0];
   const int col2 = 2 * col;
   const int nbreak = (int)red[17], nfree_mov = (int)red[18];
+  if (lane < col) {
+    const S ps = (S)red[9 + lane];
+    st->p[lane + 1] = (S)red[1 + lane];
+    st->p[col + lane + 1] = theta != S(1) ? ps * theta : ps;
+  }
   if (lane == 0) {
-    #pragma unroll 1
-    for (int j = 1; j <= col; j++) {
-      st->p[j] = (S)red[j];
-      st->p[col + j] = (S)red[8 + j];
-    }
-    if (theta != S(1))
-      #pragma unroll 1
-      for (int j = col + 1; j <= col2; j++) st->p[j] *= theta;
     st->nbreak = nbreak;
     st->nfree_mov = nfree_mov;
     st->bnded = red[19] > 0.0 ? 0 : 1;
@@ -302,9 +363,7 @@ __device__ void gcp_epilogue(DevState<S>* st, const double* red, int col, SmallW
     }
     return;
   }
-  if (lane == 0)
-    #pragma unroll 1
-    for (int j = 1; j <= col2; j++) st->c[j] = 0;
+  if (lane < col2) st->c[lane + 1] = 0;
   S f2 = -theta * f1;
   const S f2org = f2;
   if (col > 0) {
@@ -346,9 +405,8 @@ __device__ void gcp_epilogue(DevState<S>* st, const double* red, int col, SmallW
   if (lane == 0) {
     st->dtm = dtm;
     st->tsum = st->tsum + dtm;
-    #pragma unroll 1
-    for (int j = 1; j <= col2; j++) st->c[j] += dtm * st->p[j];
   }
+  if (lane < col2) st->c[lane + 1] += dtm * st->p[lane + 1];
   __syncwarp();
   if (col > 0) {
     const int info = wbmv(st->sy, st->wt, col, st->c, st->mc, sw.work, lane);  // cmprlb's M c (852)
@@ -437,9 +495,9 @@ __device__ __forceinline__ void gcp_scan_pass(const Ctx<R, H, S>& c, CtaPos cp, 
   double lo[1] = {0.0}, sd[NS];
   MinPair mn[NM] = {bp.pair()};
   sums_to_double(s, sd);
-  if (!c.epi_only) cta_reduce_to_row<CONS + 32, NS, NX, NM, 0>(sd, xm, mn, lo, c.part, W, cp.rank, cp.count);
+  if (!c.epi_only) cta_reduce_to_row<cta_threads(CONS), NS, NX, NM, 0>(sd, xm, mn, lo, c.part, W, cp.rank, cp.count);
   __shared__ double red[W];
-  if (!pass_fold<CONS + 32>(c, cp, W, NS, NX, NM, red)) return;
+  if (!pass_fold<cta_threads(CONS)>(c, cp, W, NS, NX, NM, red)) return;
   __shared__ SmallWork<S> sw;
   epilogue_on_shared_warp<S>(st, [&](DevState<S>* st, int lane) {
     gcp_epilogue<S>(st, red, col, sw, lane);
@@ -447,7 +505,7 @@ __device__ __forceinline__ void gcp_scan_pass(const Ctx<R, H, S>& c, CtaPos cp, 
 }
 
 template <typename R, typename H, typename S, int CONS>
-__global__ void __launch_bounds__(CONS + 32) k_gcp_scan(Ctx<R, H, S> c,
+__global__ void __launch_bounds__(cta_threads(CONS)) k_gcp_scan(Ctx<R, H, S> c,
     const R* __restrict__ x, const R* __restrict__ g) {
   gcp_scan_pass<R, H, S, CONS>(c, cta_here(), c.stages, x, g);
 }
@@ -474,6 +532,85 @@ __host__ __device__ inline void corr_map(int q, int& kind, int& a, int& b) {
     kind = 3;
     a = b = 0;
   }
+}
+
+// The free-set pass's epilogue, run by the 32 lanes of a warp on the shared copy of the state:
+// red is the folded row of the pass.
+template <typename S>
+__device__ __noinline__ void freev_epilogue(const double* red, int uncon, int lane) {
+  DevState<S>* st = epi_state<S>();
+  SmallWork<S>& sw = epi_scratch<S>().sw;
+  const int col = st->col;
+  const bool updatd = st->updatd != 0;
+  const S theta = st->theta;
+  constexpr int NA = 2 * kMaxM + 5, NB = 2 * kMaxM, NC = 2 * kMaxM, NS = NA + NB + NC;
+  // epilogue: freev's counts and wrk (1143-1161), formk (907-1103), subsm's K solves
+  // (1459-1471); lane 0 writes the scalars, the matrix work is shared out over the warp
+  if (lane == 0) {
+    const int nfree = (int)red[16];
+    if (!uncon) {
+      st->nfree = nfree;
+      st->nenter = (int)red[17];
+      st->nleave = (int)red[18];
+      st->wrk = (st->nleave > 0 || st->nenter > 0 || updatd) ? 1 : 0;
+    } else {
+      st->wrk = updatd ? 1 : 0;
+      st->nenter = 0;
+      st->nleave = 0;
+    }
+    st->free_hash = st->free_hash_acc;
+    st->free_hash_acc = 0;
+    st->spec_apply = 0;  // set by the direction pass when it applies an untruncated step
+    st->at_lower = (unsigned long long)red[19];
+    st->at_upper = (unsigned long long)red[20];
+    st->subsm_active = (st->nfree != 0 && col != 0) ? 1 : 0;
+  }
+  __syncwarp();
+  if (!st->subsm_active) return;
+  if (st->wrk) {
+    FormkSums<S>& fs = sw.fs;
+    if (lane < kMaxM) {
+      const int j = lane;
+      fs.yy_new[j] = (S)red[NA + j];
+      fs.sy_col[j] = (S)red[NA + kMaxM + j];
+      fs.ss_new[j] = (S)red[NA + NB + j];
+      fs.sy_row[j] = (S)red[NA + NB + kMaxM + j];
+    }
+    // (the inverse of corr_map)
+#pragma unroll
+    for (int q = lane; q < kMaxM * kMaxM; q += 32) {
+      const int a = q / kMaxM, b = q % kMaxM;
+      if (b <= a) {
+        fs.dyy[a][b] = (S)red[NS + a * (a + 1) / 2 + b];
+        fs.dss[a][b] = (S)red[NS + 36 + a * (a + 1) / 2 + b];
+      }
+      fs.dsy[a][b] = (S)red[NS + 72 + q];
+    }
+    __syncwarp();
+    const int info = wformk<S>(st->m, col, st->updatd, st->iupdat, theta, st->sy, st->wn,
+                               st->wn1, fs, sw.wm, epi_scratch<S>().snap, lane);
+    if (info != 0) {
+      if (lane == 0) st->internal_fail = info;
+      return;
+    }
+  }
+  S* wv = sw.wv;
+  if (lane < col) {
+    const int j = lane + 1;
+    wv[j] = (S)red[j - 1];
+    wv[col + j] = theta * (S)red[8 + j - 1];
+  }
+  __syncwarp();
+  const int info = wdiag_zero(st->wn, 2 * kMaxM, 2 * col, lane);
+  if (info != 0) {
+    if (lane == 0) st->internal_fail = info;
+    return;
+  }
+  wdtrsl11(st->wn, 2 * kMaxM, 2 * col, wv, lane);
+  if (lane < col) wv[lane + 1] = -wv[lane + 1];
+  __syncwarp();
+  wdtrsl1(st->wn, 2 * kMaxM, 2 * col, wv, lane);  // the same diagonal: no zero
+  if (lane < 2 * col) st->wv[lane + 1] = wv[lane + 1];
 }
 
 template <typename R, typename H, typename S, int CONS>
@@ -519,6 +656,22 @@ __device__ __forceinline__ void freev_formk_pass(const Ctx<R, H, S>& c, CtaPos c
   static_assert(!kOneRole || CONS == kTile, "one element per consumer thread and tile");
   constexpr int kRole0Warps = kOneRole ? CONS / 32 : 8, kRole12Warps = 4;
   constexpr int NA = 2 * kMaxM + 5, NB = 2 * kMaxM, NC = 2 * kMaxM;
+  constexpr int NS = NA + NB + NC;
+  constexpr int W = NS + 32 * kLaneOwned;
+  __shared__ double red[W];
+  auto warm = [&](int lane) {
+    if (!worth_warming(n, cp)) return;
+    warm_state<S>(lane);
+    for (int k = lane; k < W; k += 32) red[k] = 0.0;
+    __syncwarp();
+    if (lane == 0) {
+      red[16] = 1.0;           // free variables
+      red[NA + 1] = 1.0;       // the new row's diagonals
+      red[NA + NB + 1] = 1.0;
+    }
+    __syncwarp();
+    freev_epilogue<S>(red, 0, lane);
+  };
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int role = warp < kRole0Warps ? 0
                  : kOneRole ? 3
@@ -803,7 +956,7 @@ __device__ __forceinline__ void freev_formk_pass(const Ctx<R, H, S>& c, CtaPos c
       }
     };
     auto stream_tiles = [&](auto fast) {
-    run_stages<CONS>(ss, n, stages, dyn, reinterpret_cast<uint64_t*>(dyn + (size_t)stages * cap),
+    run_stages<CONS, true>(ss, n, stages, dyn, reinterpret_cast<uint64_t*>(dyn + (size_t)stages * cap),
                      &st->device_error, cp, [&](const unsigned char* buf, long long t, int valid,
                                             auto release) {
       if constexpr (kOneRole) {
@@ -819,7 +972,7 @@ __device__ __forceinline__ void freev_formk_pass(const Ctx<R, H, S>& c, CtaPos c
           rowprod(buf, valid, rt + h * 32 * kRole12Warps);
       }
       release();
-    });
+    }, warm);
     };
     if constexpr (kOneRole) {
       if (kFull && !uncon && track && need_row && !c.hash_free)
@@ -837,9 +990,7 @@ __device__ __forceinline__ void freev_formk_pass(const Ctx<R, H, S>& c, CtaPos c
 
   // CTA row: [ role 0: 16 sums + 5 counts | role 1: 16 | role 2: 16 | corrections ];
   // every column is summed over the warps in warp order (fixed)
-  constexpr int NS = NA + NB + NC;
-  constexpr int W = NS + 32 * kLaneOwned;
-  constexpr int kAllWarps = CONS / 32 + 1;
+  constexpr int kAllWarps = cta_threads(CONS) / 32;
   if (!c.epi_only) {
     __shared__ double wsum[kAllWarps][NS];
     for (int k = lane; k < NS; k += 32) wsum[warp][k] = 0.0;
@@ -875,7 +1026,7 @@ __device__ __forceinline__ void freev_formk_pass(const Ctx<R, H, S>& c, CtaPos c
     }
     __syncthreads();
     double* row = c.part + cp.rank;  // entry k at row[k * cp.count] (reduce.cuh)
-    for (int k = threadIdx.x; k < W; k += CONS + 32) {
+    for (int k = threadIdx.x; k < W; k += cta_threads(CONS)) {
       double a = 0.0;
       if (k < NS) {
         for (int w = 0; w < kAllWarps; w++) a += wsum[w][k];
@@ -885,82 +1036,14 @@ __device__ __forceinline__ void freev_formk_pass(const Ctx<R, H, S>& c, CtaPos c
       row[(size_t)k * cp.count] = a;
     }
   }
-  __shared__ double red[W];
-  if (!pass_fold<CONS + 32>(c, cp, W, W, 0, 0, red, &st->free_hash_acc)) return;
-  __shared__ SmallWork<S> sw;
-  __shared__ S wn1_snap[4 * kMaxM * kMaxM];
-  epilogue_on_shared_warp<S>(st, [&](DevState<S>* st, int lane) {
-    // epilogue: freev's counts and wrk (1143-1161), formk (907-1103), subsm's K solves
-    // (1459-1471); lane 0 writes the scalars, the matrix work is shared out over the warp
-    if (lane == 0) {
-      const int nfree = (int)red[16];
-      if (!uncon) {
-        st->nfree = nfree;
-        st->nenter = (int)red[17];
-        st->nleave = (int)red[18];
-        st->wrk = (st->nleave > 0 || st->nenter > 0 || updatd) ? 1 : 0;
-      } else {
-        st->wrk = updatd ? 1 : 0;
-        st->nenter = 0;
-        st->nleave = 0;
-      }
-      st->free_hash = st->free_hash_acc;
-      st->free_hash_acc = 0;
-      st->spec_apply = 0;  // set by the direction pass when it applies an untruncated step
-      st->at_lower = (unsigned long long)red[19];
-      st->at_upper = (unsigned long long)red[20];
-      st->subsm_active = (st->nfree != 0 && col != 0) ? 1 : 0;
-    }
-    __syncwarp();
-    if (!st->subsm_active) return;
-    if (st->wrk) {
-      FormkSums<S>& fs = sw.fs;
-      if (lane < kMaxM) {
-        const int j = lane;
-        fs.yy_new[j] = (S)red[NA + j];
-        fs.sy_col[j] = (S)red[NA + kMaxM + j];
-        fs.ss_new[j] = (S)red[NA + NB + j];
-        fs.sy_row[j] = (S)red[NA + NB + kMaxM + j];
-      }
-      for (int q = lane; q < 32 * kLaneOwned; q += 32) {
-        int kind, a, b;
-        corr_map(q, kind, a, b);
-        if (kind >= 3) continue;
-        const S v = (S)red[NS + q];
-        if (kind == 0) fs.dyy[a][b] = v;
-        if (kind == 1) fs.dss[a][b] = v;
-        if (kind == 2) fs.dsy[a][b] = v;
-      }
-      __syncwarp();
-      const int info = wformk<S>(st->m, col, st->updatd, st->iupdat, theta, st->sy, st->wn,
-                                 st->wn1, fs, sw.wm, wn1_snap, lane);
-      if (info != 0) {
-        if (lane == 0) st->internal_fail = info;
-        return;
-      }
-    }
-    S* wv = sw.wv;
-    if (lane < col) {
-      const int j = lane + 1;
-      wv[j] = (S)red[j - 1];
-      wv[col + j] = theta * (S)red[8 + j - 1];
-    }
-    __syncwarp();
-    const int info = wdiag_zero(st->wn, 2 * kMaxM, 2 * col, lane);
-    if (info != 0) {
-      if (lane == 0) st->internal_fail = info;
-      return;
-    }
-    wdtrsl11(st->wn, 2 * kMaxM, 2 * col, wv, lane);
-    if (lane < col) wv[lane + 1] = -wv[lane + 1];
-    __syncwarp();
-    wdtrsl1(st->wn, 2 * kMaxM, 2 * col, wv, lane);  // the same diagonal: no zero
-    if (lane < 2 * col) st->wv[lane + 1] = wv[lane + 1];
+  if (!pass_fold<cta_threads(CONS)>(c, cp, W, W, 0, 0, red, &st->free_hash_acc)) return;
+  epilogue_on_shared_warp<S>(st, [&](DevState<S>*, int lane) {
+    freev_epilogue<S>(red, uncon, lane);
   });
 }
 
 template <typename R, typename H, typename S, int CONS>
-__global__ void __launch_bounds__(CONS + 32) k_freev_formk(Ctx<R, H, S> c,
+__global__ void __launch_bounds__(cta_threads(CONS)) k_freev_formk(Ctx<R, H, S> c,
     const R* __restrict__ x, const R* __restrict__ g) {
   freev_formk_pass<R, H, S, CONS>(c, cta_here(), c.stages, x, g);
 }
@@ -1230,10 +1313,10 @@ __device__ __forceinline__ void subsm_dir_pass(const Ctx<R, H, S>& c, CtaPos cp,
   double xm[1] = {s_projected ? 1.0 : 0.0}, ldum[1] = {0.0}, sld[2];
   MinPair mn[2] = {mb.pair(), ms.pair()};
   sums_to_double(sl, sld);
-  if (!c.epi_only) cta_reduce_to_row<CONS + 32, 2, 1, 2, 0>(sld, xm, mn, ldum, c.part, W, cp.rank, cp.count);
+  if (!c.epi_only) cta_reduce_to_row<cta_threads(CONS), 2, 1, 2, 0>(sld, xm, mn, ldum, c.part, W, cp.rank, cp.count);
   __shared__ double red[W];
   __shared__ double rl[3];
-  if (!pass_fold<CONS + 32>(c, cp, W, 2, 1, 2, red)) return;
+  if (!pass_fold<cta_threads(CONS)>(c, cp, W, 2, 1, 2, red)) return;
   epilogue_on_shared<S>(st, [&](DevState<S>* st) {
     // the 3.0 step keeps the projected point when it gives a descent direction from x
     // (g'd <= 0 over the written z); otherwise, and always with the 2.1 step, the step is
@@ -1262,7 +1345,7 @@ __device__ __forceinline__ void subsm_dir_pass(const Ctx<R, H, S>& c, CtaPos cp,
 }
 
 template <typename R, typename H, typename S, int CONS>
-__global__ void __launch_bounds__(CONS + 32) k_subsm_dir(Ctx<R, H, S> c,
+__global__ void __launch_bounds__(cta_threads(CONS)) k_subsm_dir(Ctx<R, H, S> c,
     const R* __restrict__ x, const R* __restrict__ g, R* __restrict__ z) {
   subsm_dir_pass<R, H, S, CONS>(c, cta_here(), c.stages, x, g, z);
 }
@@ -1337,9 +1420,9 @@ __device__ __forceinline__ void subsm_apply_pass(const Ctx<R, H, S>& c, CtaPos c
   double xdum[1] = {0.0}, ldum[1] = {0.0}, sd[2];
   MinPair mn[1] = {ms.pair()};
   sums_to_double(s, sd);
-  if (!c.epi_only) cta_reduce_to_row<CONS + 32, 2, 0, 1, 0>(sd, xdum, mn, ldum, c.part, W, cp.rank, cp.count);
+  if (!c.epi_only) cta_reduce_to_row<cta_threads(CONS), 2, 0, 1, 0>(sd, xdum, mn, ldum, c.part, W, cp.rank, cp.count);
   __shared__ double red[W];
-  if (!pass_fold<CONS + 32>(c, cp, W, 2, 0, 1, red)) return;
+  if (!pass_fold<cta_threads(CONS)>(c, cp, W, 2, 0, 1, red)) return;
   epilogue_on_shared<S>(st, [&](DevState<S>* st) {
 
     lnsrlb_start<S>(st, red);
@@ -1347,7 +1430,7 @@ __device__ __forceinline__ void subsm_apply_pass(const Ctx<R, H, S>& c, CtaPos c
 }
 
 template <typename R, typename H, typename S, int CONS>
-__global__ void __launch_bounds__(CONS + 32) k_subsm_apply(Ctx<R, H, S> c,
+__global__ void __launch_bounds__(cta_threads(CONS)) k_subsm_apply(Ctx<R, H, S> c,
     const R* __restrict__ x, const R* __restrict__ g, R* __restrict__ z) {
   subsm_apply_pass<R, H, S, CONS>(c, cta_here(), c.stages, x, g, z);
 }
@@ -1433,47 +1516,64 @@ __device__ int post_scalar(DevState<S>* st, const double* red, S f, int force_ac
   st->updatd = 1;
   st->iupdat = st->iupdat + 1;
   const int m = st->m;
-  int shifted = 0;
   if (st->iupdat <= m) {
     st->col = st->iupdat;
     st->itail = (st->head + st->iupdat - 2) % m + 1;
   } else {
     st->itail = st->itail % m + 1;
     st->head = st->head % m + 1;
-    shifted = 1;
   }
   const int old = st->phys[st->itail];
   st->phys[st->itail] = st->spare;
   st->spare = old;
   st->theta = st->rr / dr;
-  const int ncol = st->col;
-  constexpr int ld = kMaxM;
-  if (st->iupdat > m) {
-    #pragma unroll 1
-    for (int j = 1; j <= ncol - 1; j++) {
-      #pragma unroll 1
-      for (int i = 1; i <= j; i++) LB_AT(st->ss, ld, i, j) = LB_AT(st->ss, ld, i + 1, j + 1);
-      #pragma unroll 1
-      for (int i = j; i <= ncol - 1; i++) LB_AT(st->sy, ld, i, j) = LB_AT(st->sy, ld, i + 1, j + 1);
-    }
-  }
-  #pragma unroll 1
-  for (int j = 1; j <= ncol - 1; j++) {
-    LB_AT(st->sy, ld, ncol, j) = (S)red[3 + j - 1 + shifted];
-    LB_AT(st->ss, ld, j, ncol) = (S)red[11 + j - 1 + shifted];
-  }
-  LB_AT(st->ss, ld, ncol, ncol) = (sstp == S(1)) ? st->dtd : sstp * sstp * st->dtd;
-  LB_AT(st->sy, ld, ncol, ncol) = dr;
   return 2;
 }
+// matupd's small matrices (1341-1387): S'S (upper triangle) and S'Y (lower) lose the oldest
+// pair's row and column when the ring was full, and gain the new pair's.
 template <typename S>
-__device__ bool post_epilogue(DevState<S>* st, const double* red, S f, int force_accept,
-                              int lane) {
+__device__ __forceinline__ void matupd_small(DevState<S>* st, const double* red, int lane) {
+  constexpr int ld = kMaxM;
+  const int ncol = st->col, shifted = st->iupdat > st->m ? 1 : 0;
+  const S sstp = st->stp;
+  if (shifted) {
+    S oss[2], osy[2];
+#pragma unroll
+    for (int w = 0; w < 2; w++) {
+      const int q = lane + 32 * w, i = q / kMaxM + 1, j = q % kMaxM + 1;
+      const bool in = i < ncol && j < ncol;
+      oss[w] = in ? LB_AT(st->ss, ld, i + 1, j + 1) : S(0);
+      osy[w] = in ? LB_AT(st->sy, ld, i + 1, j + 1) : S(0);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int w = 0; w < 2; w++) {
+      const int q = lane + 32 * w, i = q / kMaxM + 1, j = q % kMaxM + 1;
+      const bool in = i < ncol && j < ncol;
+      if (in && i <= j) LB_AT(st->ss, ld, i, j) = oss[w];
+      if (in && i >= j) LB_AT(st->sy, ld, i, j) = osy[w];
+    }
+    __syncwarp();
+  }
+  if (lane < ncol - 1) {
+    LB_AT(st->sy, ld, ncol, lane + 1) = (S)red[3 + lane + shifted];
+    LB_AT(st->ss, ld, lane + 1, ncol) = (S)red[11 + lane + shifted];
+  }
+  if (lane == ncol - 1) {
+    LB_AT(st->ss, ld, ncol, ncol) = (sstp == S(1)) ? st->dtd : sstp * sstp * st->dtd;
+    LB_AT(st->sy, ld, ncol, ncol) = st->dr;
+  }
+  __syncwarp();
+}
+template <typename S>
+__device__ __forceinline__ bool post_epilogue(const double* red, S f, int force_accept, int lane) {
+  DevState<S>* st = epi_state<S>();
   int r = 0;
   if (lane == 0) r = post_scalar<S>(st, red, f, force_accept);
   r = __shfl_sync(kFullMask, r, 0);
   __syncwarp();
   if (r == 2) {
+    matupd_small(st, red, lane);
     const int info = wformt<S>(st->wt, st->sy, st->ss, st->col, st->theta, lane);
     if (lane == 0 && info != 0) st->internal_fail = info;
     __syncwarp();
@@ -1509,7 +1609,8 @@ __device__ __forceinline__ void post_eval_pass(const Ctx<R, H, S>& c, CtaPos cp,
   H* ysp = c.wy + (size_t)st->spare * (size_t)c.ld;
   H* ssp = c.ws + (size_t)st->spare * (size_t)c.ld;
   // sums: [0] g'd, [1] |xold - x|^2, [2] y'y, [3..10] s'y_j, [11..18] s_j's; max: |proj g|
-  constexpr int NS = 19, NX = 1;
+  constexpr int NS = 19, NX = 1, W = NS + NX;
+  __shared__ double red[W];
   using A = typename AccOf<S>::type;
   A s[NS], xa = A(0);
 #pragma unroll
@@ -1573,20 +1674,18 @@ __device__ __forceinline__ void post_eval_pass(const Ctx<R, H, S>& c, CtaPos cp,
       ysp[i] = HistTraits<H>::from(y);
     });
   });
-  constexpr int W = NS + NX;
   MinPair mdum[1] = {MinPair{0.0, 0}};
   double ldum[1] = {0.0}, sd[NS], xm[NX] = {(double)xa};
   sums_to_double(s, sd);
-  if (!c.epi_only) cta_reduce_to_row<CONS + 32, NS, NX, 0, 0>(sd, xm, mdum, ldum, c.part, W, cp.rank, cp.count);
-  __shared__ double red[W];
-  if (!pass_fold<CONS + 32>(c, cp, W, NS, NX, 0, red)) return;
-  epilogue_on_shared_warp<S>(st, [&](DevState<S>* st, int lane) {
-    post_epilogue<S>(st, red, f, force_accept, lane);
+  if (!c.epi_only) cta_reduce_to_row<cta_threads(CONS), NS, NX, 0, 0>(sd, xm, mdum, ldum, c.part, W, cp.rank, cp.count);
+  if (!pass_fold<cta_threads(CONS)>(c, cp, W, NS, NX, 0, red)) return;
+  epilogue_on_shared_warp<S>(st, [&](DevState<S>*, int lane) {
+    post_epilogue<S>(red, f, force_accept, lane);
   });
 }
 
 template <typename R, typename H, typename S, int CONS>
-__global__ void __launch_bounds__(CONS + 32) k_post_eval(Ctx<R, H, S> c,
+__global__ void __launch_bounds__(cta_threads(CONS)) k_post_eval(Ctx<R, H, S> c,
     const R* __restrict__ t, const R* __restrict__ z, const R* __restrict__ xt,
     const R* __restrict__ gt, const R* __restrict__ go, S f, int force_accept) {
   post_eval_pass<R, H, S, CONS>(c, cta_here(), c.stages, t, z, xt, gt, go, f, force_accept);
@@ -1716,6 +1815,59 @@ __device__ __forceinline__ A stored_value(R v) {
   }
 }
 
+// The fused pass's epilogue, run by the 32 lanes of a warp on the shared copy of the state: red
+// is the folded row of the pass.
+template <typename S>
+__device__ __noinline__ void post_gcp_epilogue(const double* red, S f, int force_accept, int lane) {
+  DevState<S>* st = epi_state<S>();
+  EpiScratch<S>& x = epi_scratch<S>();
+  SmallWork<S>& sw = x.sw;
+  double* rp = x.rp;
+  double* rg = x.rg;
+  constexpr int NP = 19, NG = 21, NS = NP + NG;
+  const int col_old = st->col;
+  if (lane <= NP) rp[lane] = red[lane < NP ? lane : NS];
+  if (lane == 0) st->spec_gcp = 0;
+  __syncwarp();
+  if (!post_epilogue<S>(rp, f, force_accept, lane) || st->internal_fail != 0) return;
+  // the next iteration's loop top and cauchy epilogue (279-284, 702-747) at the accepted x
+  if (lane == 0) begin_state(st, 0);
+  __syncwarp();
+  if (st->uncon_branch) {
+    if (lane == 0) st->spec_gcp = 1;
+    return;
+  }
+  const int ncol = st->col;
+  {
+    const double* g = red + NP;
+    const int shifted = (st->updatd && st->iupdat > st->m) ? 1 : 0;
+    if (lane < kMaxM) {
+      const int j = lane + 1;
+      double ry = 0.0, rs = 0.0;
+      if (!st->updatd ? j <= col_old : j <= ncol - 1) {
+        ry = g[j + shifted];
+        rs = g[8 + j + shifted];
+      } else if (st->updatd && j == ncol) {
+        ry = g[17];
+        rs = g[18];
+      }
+      rg[j] = ry;
+      rg[8 + j] = rs;
+    }
+    if (lane == 0) {
+      rg[0] = g[0];
+      rg[17] = g[19];
+      rg[18] = g[20];
+      rg[19] = red[NS + 1];
+      rg[20] = red[NS + 2];
+      rg[21] = red[NS + 3];
+    }
+  }
+  __syncwarp();
+  gcp_epilogue<S>(st, rg, ncol, sw, lane);
+  if (lane == 0) st->spec_gcp = 1;
+}
+
 // ------------------------------------------------------------------------------------
 // E+A: the post-evaluation pass fused with the next iteration's Cauchy-point scan, for
 // problems with bounds.  Two warp roles cover every tile:
@@ -1771,7 +1923,22 @@ __device__ __forceinline__ void post_gcp_pass(const Ctx<R, H, S>& c, CtaPos cp, 
   //   position, [17] / [18] y'(-g) / s'(-g) of the new pair, [19] nbreak, [20] movable
   //   without breakpoint; xmx: any of those with g != 0; mn: smallest breakpoint.
   //   kOneRole: role G's sums in accg, its xmx in xmxg.
-  constexpr int NP = 19, NG = 21;
+  constexpr int NP = 19, NG = 21, NS = NP + NG, W = NS + 2 + 2;
+  __shared__ double red[W];
+  auto warm = [&](int lane) {
+    if (!worth_warming(n, cp)) return;
+    warm_state<S>(lane);
+    for (int k = lane; k < W; k += 32) red[k] = 0.0;
+    __syncwarp();
+    if (lane == 0) {
+      red[2] = 1.0;        // y'y
+      red[NP] = 1.0;       // a movable variable, its breakpoint beyond the minimum
+      red[NP + 19] = 1.0;
+      red[NS + 2] = 4.0;
+    }
+    __syncwarp();
+    post_gcp_epilogue<S>(red, S(0), 0, lane);
+  };
   A acc[NG];
 #pragma unroll
   for (int k = 0; k < NG; k++) acc[k] = A(0);
@@ -1946,7 +2113,7 @@ __device__ __forceinline__ void post_gcp_pass(const Ctx<R, H, S>& c, CtaPos cp, 
       }
     };
     auto stream_tiles = [&](auto fast) {
-    run_stages<CONS>(ss, n, stages, dyn,
+    run_stages<CONS, true>(ss, n, stages, dyn,
                      reinterpret_cast<uint64_t*>(dyn + (size_t)stages * cap), &st->device_error, cp,
                      [&](const unsigned char* buf, long long tt, int valid, auto release) {
       if constexpr (kOneRole) {
@@ -1960,7 +2127,7 @@ __device__ __forceinline__ void post_gcp_pass(const Ctx<R, H, S>& c, CtaPos cp, 
         for (int h = 0; h < kTile / kRoleThreads; h++) gcp_elem(buf, tt, valid, rt + h * kRoleThreads);
       }
       release();
-    });
+    }, warm);
     };
     if constexpr (kOneRole) {
       if (kFull && unit && xt_is_z)
@@ -1972,8 +2139,7 @@ __device__ __forceinline__ void post_gcp_pass(const Ctx<R, H, S>& c, CtaPos cp, 
     }
   });
   // CTA row: [ role P sums (19) | role G sums (21) | role P max | role G max | min pair ]
-  constexpr int NS = NP + NG, W = NS + 2 + 2;
-  constexpr int kAllWarps = CONS / 32 + 1;
+  constexpr int kAllWarps = cta_threads(CONS) / 32;
   if (!c.epi_only) {
     __shared__ double wsum[kAllWarps][W];
     for (int k = lane; k < W; k += 32) wsum[warp][k] = 0.0;
@@ -2005,7 +2171,7 @@ __device__ __forceinline__ void post_gcp_pass(const Ctx<R, H, S>& c, CtaPos cp, 
     }
     __syncthreads();
     double* row = c.part + cp.rank;  // entry k at row[k * cp.count] (reduce.cuh)
-    for (int k = threadIdx.x; k < W; k += CONS + 32) {
+    for (int k = threadIdx.x; k < W; k += cta_threads(CONS)) {
       if (k < NS) {
         double a = 0.0;
         for (int w = 0; w < kAllWarps; w++) a += wsum[w][k];
@@ -2023,62 +2189,14 @@ __device__ __forceinline__ void post_gcp_pass(const Ctx<R, H, S>& c, CtaPos cp, 
       }
     }
   }
-  __shared__ double red[W];
-  if (!pass_fold<CONS + 32>(c, cp, W, NS, 2, 1, red)) return;
-  __shared__ SmallWork<S> sw;
-  __shared__ double rp[NP + 1], rg[22];  // epilogue temporaries (shared, as all of them)
-  epilogue_on_shared_warp<S>(st, [&](DevState<S>* st, int lane) {
-    if (lane == 0) {
-      for (int k = 0; k < NP; k++) rp[k] = red[k];
-      rp[NP] = red[NS];
-      st->spec_gcp = 0;
-    }
-    __syncwarp();
-    const int col_old = col;
-    if (!post_epilogue<S>(st, rp, f, force_accept, lane) || st->internal_fail != 0) return;
-    // the next iteration's loop top and cauchy epilogue (279-284, 702-747) at the accepted x
-    if (lane == 0) begin_state(st, 0);
-    __syncwarp();
-    if (st->uncon_branch) {
-      if (lane == 0) st->spec_gcp = 1;
-      return;
-    }
-    const int ncol = st->col;
-    if (lane == 0) {
-      const double* g = red + NP;
-      const int shifted = (st->updatd && st->iupdat > st->m) ? 1 : 0;
-      rg[0] = g[0];
-      for (int j = 1; j <= kMaxM; j++) {
-        rg[j] = 0.0;
-        rg[8 + j] = 0.0;
-      }
-      if (!st->updatd) {
-        for (int j = 1; j <= col_old; j++) {
-          rg[j] = g[j];
-          rg[8 + j] = g[8 + j];
-        }
-      } else {
-        for (int j = 1; j <= ncol - 1; j++) {
-          rg[j] = g[j + shifted];
-          rg[8 + j] = g[8 + j + shifted];
-        }
-        rg[ncol] = g[17];
-        rg[8 + ncol] = g[18];
-      }
-      rg[17] = g[19];
-      rg[18] = g[20];
-      rg[19] = red[NS + 1];
-      rg[20] = red[NS + 2];
-      rg[21] = red[NS + 3];
-    }
-    __syncwarp();
-    gcp_epilogue<S>(st, rg, ncol, sw, lane);
-    if (lane == 0) st->spec_gcp = 1;
+  if (!pass_fold<cta_threads(CONS)>(c, cp, W, NS, 2, 1, red)) return;
+  epilogue_on_shared_warp<S>(st, [&](DevState<S>*, int lane) {
+    post_gcp_epilogue<S>(red, f, force_accept, lane);
   });
 }
 
 template <typename R, typename H, typename S, int CONS>
-__global__ void __launch_bounds__(CONS + 32) k_post_gcp(Ctx<R, H, S> c,
+__global__ void __launch_bounds__(cta_threads(CONS)) k_post_gcp(Ctx<R, H, S> c,
     const R* __restrict__ t, const R* __restrict__ z, const R* __restrict__ xt,
     const R* __restrict__ gt, const R* __restrict__ go, S f, int force_accept) {
   post_gcp_pass<R, H, S, CONS>(c, cta_here(), c.stages, t, z, xt, gt, go, f, force_accept);

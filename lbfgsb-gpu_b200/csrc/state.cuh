@@ -72,11 +72,18 @@ struct DevState {
 // threads store the copy back.  epilogue_on_shared runs f(st) on thread 0;
 // epilogue_on_shared_warp runs f(st, lane) on the 32 lanes of warp 0, for epilogues whose
 // matrix algebra is shared out over a warp (warp_small.cuh).
+// The copy lies in one shared variable per kernel (epi_state), so that an epilogue that is a
+// function of its own addresses it as shared memory.
+template <typename S>
+__device__ __forceinline__ DevState<S>* epi_state() {
+  static_assert(sizeof(DevState<S>) % 4 == 0, "the state is copied in 4-byte words");
+  __shared__ __align__(16) unsigned int words[sizeof(DevState<S>) / 4];
+  return reinterpret_cast<DevState<S>*>(words);
+}
 template <bool kWarp, typename S, typename F>
 __device__ __forceinline__ void epilogue_in_shared(DevState<S>* st, F&& f) {
-  static_assert(sizeof(DevState<S>) % 4 == 0, "the state is copied in 4-byte words");
   constexpr int kWords = (int)(sizeof(DevState<S>) / 4);
-  __shared__ __align__(16) unsigned int words[kWords];
+  unsigned int* words = reinterpret_cast<unsigned int*>(epi_state<S>());
   const unsigned int* src = reinterpret_cast<const unsigned int*>(st);
   for (int k = threadIdx.x; k < kWords; k += blockDim.x) words[k] = __ldcg(src + k);
   __syncthreads();

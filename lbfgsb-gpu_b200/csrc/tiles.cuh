@@ -200,8 +200,16 @@ __device__ __forceinline__ void load_tile(const StreamSet& ss, long long t, long
 
 constexpr int kMaxStages = 8;
 
-// Warp-specialised tile pipeline.  The CTA has CONSUMERS + 32 threads: the last warp is
-// the producer, which issues the copies of the CTA's tiles (tiles rank, rank + count, ...
+// Threads of a CTA of a staged pass with `consumers` consumer threads: a producer warp and an
+// idle warp after them (a fifth warp of one scheduler either way, so it costs no registers).
+__host__ __device__ constexpr int cta_threads(int consumers) { return consumers + 64; }
+
+struct NoIdleWork {
+  __device__ __forceinline__ void operator()(int) const {}
+};
+
+// Warp-specialised tile pipeline.  The CTA has cta_threads(CONSUMERS) threads: the warp after
+// the consumers is the producer, which issues the copies of the CTA's tiles (tiles rank, rank + count, ...
 // of the instance's n elements) into a ring of `stages` stage buffers; the consumer threads run
 // body(buf, t, valid) once per tile.  full[s] completes when the bytes of the tile in
 // stage s have landed; empty[s] completes when every consumer warp has finished with it.
@@ -210,12 +218,13 @@ constexpr int kMaxStages = 8;
 // call release() exactly once, with the whole warp, after its last read of the stage
 // buffer; a body that reads its data into registers first can release the stage before it
 // computes, so that the producer refills it sooner.  body must not contain block-level
-// barriers nor write the stage buffer.  Every wait is bounded; on a timeout the CTA sets
-// *err and leaves the loop (returns false).
-template <int CONSUMERS, typename Body>
+// barriers nor write the stage buffer.  With kIdle the idle warp runs idle(lane) once beside the
+// pipeline (the passes with long epilogues run the epilogue's code there, passes.cuh).  Every
+// wait is bounded; on a timeout the CTA sets *err and leaves the loop (returns false).
+template <int CONSUMERS, bool kIdle = false, typename Body, typename Idle = NoIdleWork>
 __device__ __forceinline__ bool run_stages(const StreamSet& ss, long long n, int stages,
                                            unsigned char* ring, uint64_t* bars, int* err,
-                                           CtaPos cp, Body&& body) {
+                                           CtaPos cp, Body&& body, Idle&& idle = Idle{}) {
   constexpr int kConsumerWarps = CONSUMERS / 32;
   uint64_t* full = bars;
   uint64_t* empty = bars + stages;
@@ -256,7 +265,9 @@ __device__ __forceinline__ bool run_stages(const StreamSet& ss, long long n, int
         wrapped = true;
       }
     }
-  } else {
+  } else if (kIdle && warp > kConsumerWarps) {
+    if constexpr (kIdle) idle(lane);
+  } else if (warp < kConsumerWarps) {
     // consumers
     int s = 0;
     uint32_t ph = 0;
