@@ -561,7 +561,7 @@ struct WalkCoop {
     };
   };
   S f1, f2, dtm, tsum, tj;                       // before the next key to be tested
-  int nleft, nint, all_fixed, done, stop, passed, info;
+  int nleft, nint, all_fixed, done, passed, info;
 };
 
 // Sorts the kPiece keys held one per thread (a bitonic network; partners within a warp by
@@ -746,13 +746,15 @@ __device__ void walk_records_in_order(const Ctx<R, H, S>& c, const WalkRecords<S
     pj = st->p[lane + 1];
     cj = st->c[lane + 1];
   }
-  if (threadIdx.x == 0) {
-    sm.stop = 0;
-    sm.passed = cnt;
-  }
+  if (threadIdx.x == 0) sm.passed = cnt;
   stage(0, (int)threadIdx.x, std::integral_constant<int, kWalkThreads>{});
   __syncthreads();
+  // The test's warp ends the loop through the step's barrier itself: every thread gets the same
+  // answer for the same step, however late it leaves the barrier (a flag in shared memory, read
+  // after the barrier, would be written by the next step's test before a late warp has read it).
+  bool stopped = false;
   for (int s = 0; s < nsub + 4; s++) {
+    bool stop_here = false;
     if (warp == kWalkThreads / 32 - 1) {
       if (lane == 0 && s >= 3 && s - 3 < nsub) {
         // the sum of dt, at the pace of f'
@@ -908,21 +910,23 @@ __device__ void walk_records_in_order(const Ctx<R, H, S>& c, const WalkRecords<S
             sm.dtm = 0;
           }
           if (hit >= 0) {
-            sm.stop = 1;
+            stop_here = true;
             sm.passed = base + hit;
           }
           if (hit >= 0 || last) sm.done = 1;
         }
       }
     }
-    __syncthreads();
-    if (sm.stop) break;
+    if (__syncthreads_or(stop_here)) {
+      stopped = true;
+      break;
+    }
   }
   const int passed = sm.passed;
   if (warp == 0 && lane < col2) {
-    if (sm.stop || sm.all_fixed) {
+    if (stopped || sm.all_fixed) {
       // p and c where the walk ended, from the start of that sub-batch
-      const int b = sm.stop ? passed / kSub : (cnt - 1) / kSub;
+      const int b = stopped ? passed / kSub : (cnt - 1) / kSub;
       pj = sm.ckp[b][lane];
       cj = sm.ckc[b][lane];
       for (int k = b * kSub; k < passed; k++) {
