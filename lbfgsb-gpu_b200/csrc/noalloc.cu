@@ -42,9 +42,13 @@ static __device__ __align__(256) unsigned long long g_projgr_scratch[32 + kNoAll
 // One launch of at most a few thousand variables is bound by latency (the loads, the ticket,
 // the fold), a large one by HBM.  kPer, the elements per thread, is chosen so that a small
 // call spreads over the SMs: with 16 each, in a loop, n = 65,536 ran on 16 CTAs and took
-// 16.3 us, one load round trip (two, for the bound that the sign of g selects) per element.
-// All loads of up to four elements are now issued together; both bounds are read (signs mix
-// within a 32-byte sector, so that one bound per element moves the same sectors).
+// 17.4 us (6.2 now), one load round trip (two, for the bound that the sign of g selects) per
+// element.  Two elements' loads are in flight together, behind their nbd, which is loaded one
+// step ahead: x and a bound are read only where nbd says that the variable has that bound (the
+// caller's arrays need hold nothing else), so that an unbounded variable moves 12 bytes, not 36.
+// us a call, the loop over 16 elements / both bounds read whatever nbd / this one, n = 2^25: nbd 0
+// 90 / 170 / 76, nbd 1 197 / 172 / 138, nbd 2 254 / 172 / 174; n = 4,000,000: nbd 0 11.4 / 27.5 /
+// 13.5, nbd 2 41 / 28.7 / 28.  Four elements together: 86, 141 and 174 us at 2^25.
 template <int kPer>
 __global__ void __launch_bounds__(kNoAllocThreads)
     k_projgr_noalloc(int n, const double* __restrict__ x, const double* __restrict__ g,
@@ -53,22 +57,30 @@ __global__ void __launch_bounds__(kNoAllocThreads)
   unsigned long long* ticket = scratch;
   unsigned long long* rows = scratch + 32;
   const long long base = (long long)blockIdx.x * (kPer * kNoAllocThreads) + threadIdx.x;
-  constexpr int kLoad = kPer < 4 ? kPer : 4;  // elements whose loads are in flight together
+  constexpr int kLoad = kPer < 2 ? kPer : 2;  // elements whose loads are in flight together
   double m = 0.0;
-#pragma unroll 1
-  for (int k = 0; k < kPer; k += kLoad) {
-    double xi[kLoad], gi[kLoad], li[kLoad], ui[kLoad];
-    int nb[kLoad];
+  int nb[kLoad], next[kLoad];
+  auto kinds = [&](int k) {
 #pragma unroll
     for (int q = 0; q < kLoad; q++) {
       const long long i = base + (long long)(k + q) * kNoAllocThreads;
-      const bool in = i < n;
-      xi[q] = in ? x[i] : 0.0;
-      gi[q] = in ? g[i] : 0.0;  // g = 0, nbd = 0 adds |0|
-      nb[q] = in ? nbd[i] : 0;
-      li[q] = in ? l[i] : 0.0;
-      ui[q] = in ? u[i] : 0.0;
+      next[q] = i < n ? nbd[i] : 0;
     }
+  };
+  kinds(0);
+#pragma unroll 1
+  for (int k = 0; k < kPer; k += kLoad) {
+    double xi[kLoad], gi[kLoad], li[kLoad], ui[kLoad];
+#pragma unroll
+    for (int q = 0; q < kLoad; q++) {
+      const long long i = base + (long long)(k + q) * kNoAllocThreads;
+      nb[q] = next[q];
+      gi[q] = i < n ? g[i] : 0.0;  // g = 0, nbd = 0 adds |0|
+      xi[q] = nb[q] != 0 ? x[i] : 0.0;
+      li[q] = nb[q] != 0 && nb[q] <= 2 ? l[i] : 0.0;
+      ui[q] = nb[q] >= 2 ? u[i] : 0.0;
+    }
+    if (k + kLoad < kPer) kinds(k + kLoad);
 #pragma unroll
     for (int q = 0; q < kLoad; q++) {
       double pg = gi[q];

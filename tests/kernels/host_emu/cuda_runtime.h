@@ -40,6 +40,8 @@ struct Fiber {
   int block_line = 0;  // the source line of the block barrier it waits at, 0: none
   bool in_warp = false;
   int pred = 0;  // the value it brought to its warp's or the block's vote
+  double carried[2];  // the values it brought to its warp's last two shuffles
+  int shuffles = 0;
 };
 inline std::vector<Fiber> fibers;
 inline ucontext_t scheduler;
@@ -69,6 +71,14 @@ inline unsigned warp_vote(int pred) {
   fibers[current].pred = pred;
   yield();
   return warp_mask[current / 32];
+}
+
+inline double shuffle_xor(double v, int lanes) {
+  Fiber& f = fibers[current];
+  const int slot = f.shuffles++ & 1, partner = current ^ lanes;
+  f.carried[slot] = v;
+  warp_vote(0);
+  return fibers[partner].carried[slot];
 }
 
 // Runs fn on `threads` threads of block `block`; false when barriers diverge or cannot complete.
@@ -145,6 +155,7 @@ inline void __syncwarp(unsigned = 0xffffffffu) { emu::warp_vote(0); }
 inline unsigned __ballot_sync(unsigned, int p) { return emu::warp_vote(p); }
 inline int __any_sync(unsigned, int p) { return emu::warp_vote(p) != 0; }
 inline int __all_sync(unsigned, int p) { return emu::warp_vote(p) == 0xffffffffu; }
+inline double __shfl_xor_sync(unsigned, double v, int lanes) { return emu::shuffle_xor(v, lanes); }
 inline int __ffs(unsigned m) { return __builtin_ffs((int)m); }
 inline int __popc(unsigned m) { return __builtin_popcount(m); }
 template <typename T>
@@ -176,8 +187,8 @@ inline float __fmul_rn(float a, float b) { return a * b; }
 inline float __fdiv_rn(float a, float b) { return a / b; }
 inline void __threadfence() {}
 // named by sources whose use of them no test runs
-template <typename T>
-T __shfl_xor_sync(unsigned, T, int);
+unsigned long long __shfl_xor_sync(unsigned, unsigned long long, int);
+unsigned int __shfl_xor_sync(unsigned, unsigned int, int);
 double __fma_rn(double, double, double);
 float __fmaf_rn(float, float, float);
 double __dmul_ru(double, double), __dmul_rd(double, double);

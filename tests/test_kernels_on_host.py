@@ -5,7 +5,10 @@ walk_pipeline_check: the cooperative walk's pipeline with one warp late at every
 walk as the reference's serial recurrence does, bit for bit, with all threads at the same
 barriers: stopping at the edges of its sub-batches, at the last breakpoint (bounded or not),
 with every variable fixed, with f'' at its lower limit, without a history, over several chunks,
-in double and in float."""
+in double and in float.
+
+projgr_reads_check: the projected-gradient norm must not read a bound (nor x) that nbd says is
+not there; those arrays lie on unreadable pages."""
 import os
 import re
 import subprocess
@@ -27,9 +30,9 @@ def _between(text, first, after):
     return text[a:text.index(after, a)]
 
 
-def _compile(tmp, check):
+def _compile(tmp, check, opt="-O1"):
     exe = tmp / check
-    subprocess.run(["g++", "-std=c++17", "-O1", "-ffp-contract=off", "-w", f"-I{tmp}",
+    subprocess.run(["g++", "-std=c++17", opt, "-ffp-contract=off", "-w", f"-I{tmp}",
                     f"-I{os.path.join(KERNELS, 'host_emu')}", f"-I{CSRC}",
                     os.path.join(KERNELS, check + ".cpp"), "-o", str(exe)], check=True)
     return str(exe)
@@ -53,3 +56,18 @@ def walk_exe(tmp_path_factory):
 def test_walk_pipeline(walk_exe, what, real):
     r = subprocess.run([walk_exe, real, what], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.fixture(scope="module")
+def projgr_exe(tmp_path_factory):
+    tmp = tmp_path_factory.mktemp("projgr")
+    body = _between(_source("noalloc.cu"), "constexpr int kNoAllocThreads",
+                    "// Address of the scratch on the current device")
+    (tmp / "projgr_slice.cuh").write_text("namespace lbfgsb_b200 {\n" + body + "\n}\n")
+    return _compile(tmp, "projgr_reads_check", "-O0")  # -O1 drops loads that are not used
+
+
+@pytest.mark.parametrize("per_thread", [1, 4, 16])
+def test_projgr_reads_only_bounds_that_exist(projgr_exe, per_thread):
+    r = subprocess.run([projgr_exe, str(per_thread)], capture_output=True, text=True)
+    assert r.returncode == 0, (r.returncode, r.stderr[-2000:])
