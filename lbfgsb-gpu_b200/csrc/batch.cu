@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(cta_threads(CONS)) kb_gcp_scan(BatchLaunch<R, 
   gcp_scan_pass<R, H, S, CONS>(b.table[k], cp, b.stages, nullptr, nullptr);
 }
 template <typename R, typename H, typename S, int CONS>
-__global__ void __launch_bounds__(cta_threads(CONS)) kb_freev_formk(BatchLaunch<R, H, S> b) {
+__global__ void __launch_bounds__(warming_threads(CONS)) kb_freev_formk(BatchLaunch<R, H, S> b) {
   CtaPos cp;
   const int k = batch_instance(b.first, b.count, cp);
   freev_formk_pass<R, H, S, CONS>(b.table[k], cp, b.stages, nullptr, nullptr);
@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(cta_threads(CONS)) kb_subsm_apply(BatchLaunch<
 // the post-evaluation pass with the next Cauchy scan for instances with bounds, the plain
 // one for the others (as the single-instance driver chooses)
 template <typename R, typename H, typename S, int CONS>
-__global__ void __launch_bounds__(cta_threads(CONS)) kb_post_gcp(BatchLaunch<R, H, S> b) {
+__global__ void __launch_bounds__(warming_threads(CONS)) kb_post_gcp(BatchLaunch<R, H, S> b) {
   CtaPos cp;
   const int k = batch_instance(b.first, b.count, cp);
   const Ctx<R, H, S>& c = b.table[k];
@@ -676,20 +676,20 @@ class BatchRunner {
     const int rb = (cnt + 127) / 128;
     const BatchLaunch<R, H, S> bp{table_, first_pass_, cnt, 2};
     const BatchLaunch<R, H, S> be{table_, first_elem_, cnt, 2};
-    const int thr = cta_threads(kConsWide);
+    const int thr = cta_threads(kConsWide), warming = warming_threads(kConsWide);
     CK(cudaStreamBeginCapture(s_, cudaStreamCaptureModeThreadLocal));
     kb_round<R, H, S, RK_BEGIN><<<rb, 128, 0, s_>>>(table_, cnt);
     kb_gcp_scan<R, H, S, kConsWide><<<ctas_pass_, thr, ring_bytes(2, cap_gcp_), s_>>>(bp);
     kb_walk_gather<R, H, S><<<ctas_elem_, kThreads, 0, s_>>>(be);
     kb_walk<R, H, S><<<cnt, kWalkThreads, 0, s_>>>(table_);
-    kb_freev_formk<R, H, S, kConsWide><<<ctas_pass_, thr, ring_bytes(2, cap_freev_) + freev_extra_smem<S>(), s_>>>(bp);
+    kb_freev_formk<R, H, S, kConsWide><<<ctas_pass_, warming, ring_bytes(2, cap_freev_) + freev_extra_smem<S>(), s_>>>(bp);
     kb_subsm_dir<R, H, S, kConsWide><<<ctas_pass_, thr, ring_bytes(2, cap_dir_), s_>>>(bp);
     kb_subsm_apply<R, H, S, kConsWide><<<ctas_pass_, thr, ring_bytes(2, cap_apply_), s_>>>(bp);
     kb_round<R, H, S, RK_PRE><<<rb, 128, 0, s_>>>(table_, cnt);
     kb_trial_round<R, H, S><<<ctas_elem_, 256, 0, s_>>>(be);
     objective_(user_, cnt, ids_, first_elem_, ctas_elem_, (const R* const*)ev_x_, ev_g_, ev_f_,
                ev_act_, (void*)s_);
-    kb_post_gcp<R, H, S, kConsWide><<<ctas_pass_, thr, ring_bytes(2, cap_post_), s_>>>(bp);
+    kb_post_gcp<R, H, S, kConsWide><<<ctas_pass_, warming, ring_bytes(2, cap_post_), s_>>>(bp);
     if (any_uncon_)
       kb_post_eval<R, H, S, kConsWide><<<ctas_pass_, thr, ring_bytes(2, cap_post_), s_>>>(bp);
     kb_round<R, H, S, RK_POST><<<rb, 128, 0, s_>>>(table_, cnt);

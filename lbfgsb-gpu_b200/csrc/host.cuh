@@ -375,7 +375,7 @@ static void prepare(Workspace<R, H, S>& w, Ctx<R, H, S>& c, Plan& p, int n, int 
   p.gcp = pass_cfg(k_gcp_scan<R, H, S, kConsWide>,
                    stage_capacity(StageBytes<R>::gcp, 0, m, hsz), n, cta_threads(kConsWide));
   p.freev = pass_cfg(k_freev_formk<R, H, S, kConsWide>,
-                     stage_capacity(StageBytes<R>::freev, kTile / 8, m, hsz), n, cta_threads(kConsWide),
+                     stage_capacity(StageBytes<R>::freev, kTile / 8, m, hsz), n, warming_threads(kConsWide),
                      freev_extra_smem<S>());
   p.dir = pass_cfg(k_subsm_dir<R, H, S, kConsWide>,
                    stage_capacity(StageBytes<R>::dir, 0, m, hsz), n, cta_threads(kConsWide));
@@ -384,7 +384,7 @@ static void prepare(Workspace<R, H, S>& w, Ctx<R, H, S>& c, Plan& p, int n, int 
   p.post = pass_cfg(k_post_eval<R, H, S, kConsWide>,
                     stage_capacity(StageBytes<R>::post, 0, m, hsz), n, cta_threads(kConsWide));
   p.pgcp = pass_cfg(k_post_gcp<R, H, S, kConsWide>,
-                    stage_capacity(StageBytes<R>::post, 0, m, hsz), n, cta_threads(kConsWide));
+                    stage_capacity(StageBytes<R>::post, 0, m, hsz), n, warming_threads(kConsWide));
   p.g_proj = grid_for(k_projgr<R, H, S>, n, kThreads);
   const int g_max = std::max({p.gcp.grid, p.freev.grid, p.dir.grid, p.apply.grid, p.post.grid,
                               p.pgcp.grid, p.g_proj});

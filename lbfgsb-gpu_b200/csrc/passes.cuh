@@ -281,8 +281,13 @@ __device__ __forceinline__ EpiScratch<S>& epi_scratch() {
 // path through every routine: a full ring that shifts, identity matrices, an accepted step.
 //
 // Below kWarmTiles tiles a CTA nothing is warmed: the last CTA would wait for its own warm-up, and
-// its code is still in L2 (n = 333^2, 1-2 tiles a CTA: 9% slower with the warm-up, n = 256^2 5%;
-// n = 1024^2 FP32, 13 tiles: 3% faster; 2048^2 mixed, 55 tiles: 3%).
+// its code is still in L2.  ms a solve of 14 iterations, with / without the warm-up, by tiles a
+// CTA: FP64 2: 2.21 / 2.03, 5: 2.47 / 2.43, 7: 2.66 / 2.74, 13: 3.38 / 3.60, 55: 8.02 / 8.26,
+// 221: 26.19 / 26.43; mixed 5: 2.38 / 2.32, 8: 2.57 / 2.58, 13: 2.98 / 3.03, 55: 6.74 / 7.03; FP32
+// 5: 2.22 / 2.17, 8: 2.36 / 2.37, 13: 2.64 / 2.69, 55: 5.52 / 5.74, 221: 15.75 / 15.97.
+//
+// Only these two passes have the extra warp.  In the others, where it only waited at the barriers,
+// it cost the streaming up to 2.7% (k_subsm_dir, n = 4096^2 FP64: 433 us a launch against 422).
 constexpr int kWarmTiles = 8;
 __device__ __forceinline__ bool worth_warming(int n, CtaPos cp) {
   return n / kTile >= kWarmTiles * cp.count;
@@ -990,7 +995,7 @@ __device__ __forceinline__ void freev_formk_pass(const Ctx<R, H, S>& c, CtaPos c
 
   // CTA row: [ role 0: 16 sums + 5 counts | role 1: 16 | role 2: 16 | corrections ];
   // every column is summed over the warps in warp order (fixed)
-  constexpr int kAllWarps = cta_threads(CONS) / 32;
+  constexpr int kAllWarps = warming_threads(CONS) / 32;
   if (!c.epi_only) {
     __shared__ double wsum[kAllWarps][NS];
     for (int k = lane; k < NS; k += 32) wsum[warp][k] = 0.0;
@@ -1026,7 +1031,7 @@ __device__ __forceinline__ void freev_formk_pass(const Ctx<R, H, S>& c, CtaPos c
     }
     __syncthreads();
     double* row = c.part + cp.rank;  // entry k at row[k * cp.count] (reduce.cuh)
-    for (int k = threadIdx.x; k < W; k += cta_threads(CONS)) {
+    for (int k = threadIdx.x; k < W; k += warming_threads(CONS)) {
       double a = 0.0;
       if (k < NS) {
         for (int w = 0; w < kAllWarps; w++) a += wsum[w][k];
@@ -1036,14 +1041,14 @@ __device__ __forceinline__ void freev_formk_pass(const Ctx<R, H, S>& c, CtaPos c
       row[(size_t)k * cp.count] = a;
     }
   }
-  if (!pass_fold<cta_threads(CONS)>(c, cp, W, W, 0, 0, red, &st->free_hash_acc)) return;
+  if (!pass_fold<warming_threads(CONS)>(c, cp, W, W, 0, 0, red, &st->free_hash_acc)) return;
   epilogue_on_shared_warp<S>(st, [&](DevState<S>*, int lane) {
     freev_epilogue<S>(red, uncon, lane);
   });
 }
 
 template <typename R, typename H, typename S, int CONS>
-__global__ void __launch_bounds__(cta_threads(CONS)) k_freev_formk(Ctx<R, H, S> c,
+__global__ void __launch_bounds__(warming_threads(CONS)) k_freev_formk(Ctx<R, H, S> c,
     const R* __restrict__ x, const R* __restrict__ g) {
   freev_formk_pass<R, H, S, CONS>(c, cta_here(), c.stages, x, g);
 }
@@ -2139,7 +2144,7 @@ __device__ __forceinline__ void post_gcp_pass(const Ctx<R, H, S>& c, CtaPos cp, 
     }
   });
   // CTA row: [ role P sums (19) | role G sums (21) | role P max | role G max | min pair ]
-  constexpr int kAllWarps = cta_threads(CONS) / 32;
+  constexpr int kAllWarps = warming_threads(CONS) / 32;
   if (!c.epi_only) {
     __shared__ double wsum[kAllWarps][W];
     for (int k = lane; k < W; k += 32) wsum[warp][k] = 0.0;
@@ -2171,7 +2176,7 @@ __device__ __forceinline__ void post_gcp_pass(const Ctx<R, H, S>& c, CtaPos cp, 
     }
     __syncthreads();
     double* row = c.part + cp.rank;  // entry k at row[k * cp.count] (reduce.cuh)
-    for (int k = threadIdx.x; k < W; k += cta_threads(CONS)) {
+    for (int k = threadIdx.x; k < W; k += warming_threads(CONS)) {
       if (k < NS) {
         double a = 0.0;
         for (int w = 0; w < kAllWarps; w++) a += wsum[w][k];
@@ -2189,14 +2194,14 @@ __device__ __forceinline__ void post_gcp_pass(const Ctx<R, H, S>& c, CtaPos cp, 
       }
     }
   }
-  if (!pass_fold<cta_threads(CONS)>(c, cp, W, NS, 2, 1, red)) return;
+  if (!pass_fold<warming_threads(CONS)>(c, cp, W, NS, 2, 1, red)) return;
   epilogue_on_shared_warp<S>(st, [&](DevState<S>*, int lane) {
     post_gcp_epilogue<S>(red, f, force_accept, lane);
   });
 }
 
 template <typename R, typename H, typename S, int CONS>
-__global__ void __launch_bounds__(cta_threads(CONS)) k_post_gcp(Ctx<R, H, S> c,
+__global__ void __launch_bounds__(warming_threads(CONS)) k_post_gcp(Ctx<R, H, S> c,
     const R* __restrict__ t, const R* __restrict__ z, const R* __restrict__ xt,
     const R* __restrict__ gt, const R* __restrict__ go, S f, int force_accept) {
   post_gcp_pass<R, H, S, CONS>(c, cta_here(), c.stages, t, z, xt, gt, go, f, force_accept);

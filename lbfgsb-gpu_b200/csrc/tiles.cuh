@@ -200,9 +200,10 @@ __device__ __forceinline__ void load_tile(const StreamSet& ss, long long t, long
 
 constexpr int kMaxStages = 8;
 
-// Threads of a CTA of a staged pass with `consumers` consumer threads: a producer warp and an
-// idle warp after them (a fifth warp of one scheduler either way, so it costs no registers).
-__host__ __device__ constexpr int cta_threads(int consumers) { return consumers + 64; }
+// Threads of a CTA of a staged pass with `consumers` consumer threads: a producer warp after them,
+// and in the passes that warm their epilogue (passes.cuh) an otherwise idle warp after that.
+__host__ __device__ constexpr int cta_threads(int consumers) { return consumers + 32; }
+__host__ __device__ constexpr int warming_threads(int consumers) { return consumers + 64; }
 
 struct NoIdleWork {
   __device__ __forceinline__ void operator()(int) const {}
