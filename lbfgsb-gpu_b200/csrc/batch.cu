@@ -136,13 +136,14 @@ __global__ void __launch_bounds__(kThreads) kb_setup(const Ctx<R, H, S>* table, 
   for (int k = threadIdx.x; k < words; k += kThreads) c.fbits[k] = 0u;
   if (threadIdx.x == 0) *c.ticket = 0u;
 }
-// The iterates of the finished instances into the callers' arrays, in one launch.
+// The iterates of the finished instances among the first `known` into the callers' arrays, in one
+// launch.
 template <typename R, typename H, typename S>
-__global__ void __launch_bounds__(kThreads) kb_copy_back(BatchLaunch<R, H, S> b, R* const* x_out) {
+__global__ void __launch_bounds__(kThreads) kb_copy_back(BatchLaunch<R, H, S> b, int known, R* const* x_out) {
   CtaPos cp;
   const int k = batch_instance(b.first, b.count, cp);
   const Ctx<R, H, S>& c = b.table[k];
-  if (c.st->phase != PH_DONE) return;
+  if (k >= known || c.st->phase != PH_DONE) return;
   const R* __restrict__ x = c.X[c.st->xr[0]];
   R* __restrict__ out = x_out[k];
   const long long stride = (long long)cp.count * kThreads;
@@ -423,10 +424,10 @@ class BatchRunner {
     if (dirty_) rebuild();
     std::vector<BatchRow> rows = collect((int)live_.size());
     std::vector<Inst> keep, ended;
-    for (size_t j = 0; j < live_.size(); j++) {
-      Inst& in = live_[j];
-      const BatchRow& r = rows[j];
-      if (r.device_error) throw CudaFailure{cudaErrorLaunchTimeout, "staged-tile wait", __LINE__};
+    size_t known = 0;  // the instances before the first one whose wait gave up
+    for (; known < live_.size() && !rows[known].device_error; known++) {
+      Inst& in = live_[known];
+      const BatchRow& r = rows[known];
       if (r.phase != PH_DONE) {
         keep.push_back(in);
         continue;
@@ -436,19 +437,20 @@ class BatchRunner {
       in.summary->residual_g = (R)r.res_g;
       in.summary->residual_x = (R)r.res_x;
       in.summary->residual_f = (R)r.res_f;
-      *in.status = LBFGSB_B200_OK;
       ended.push_back(in);
     }
     if (!ended.empty()) {
       const BatchLaunch<R, H, S> be{table_, first_elem_, count_, 2};
-      kb_copy_back<R, H, S><<<ctas_elem_, kThreads, 0, s_>>>(be, const_cast<R* const*>(xin_));
+      kb_copy_back<R, H, S><<<ctas_elem_, kThreads, 0, s_>>>(be, (int)known, const_cast<R* const*>(xin_));
       CK(cudaGetLastError());
       launches_++;
       for (Inst& in : ended) {
+        *in.status = LBFGSB_B200_OK;  // x is on its way
         release(in);
         finished->push_back(in);
       }
     }
+    if (known < live_.size()) throw CudaFailure{cudaErrorLaunchTimeout, "staged-tile wait", __LINE__};
     if (keep.size() != live_.size()) {
       live_.swap(keep);
       dirty_ = true;
