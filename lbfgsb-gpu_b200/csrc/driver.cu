@@ -123,7 +123,7 @@ static int solve(int n, R* x_user, const int* nbd, const R* l, const R* u,
     const PassCfg &p_gcp = p.gcp, &p_freev = p.freev, &p_dir = p.dir, &p_apply = p.apply,
                   &p_post = p.post, &p_pgcp = p.pgcp;
     const int g_proj = p.g_proj, g_elem = p.g_elem;
-    const int g_walk = walk_coop_grid<R, H, S>();
+    const int g_walk = walk_coop_grid<R, H, S>(false);
     DevState<S>& hs = *w.hs;
     // sharded: the buffers of the rank rows (shard.cuh, reduce.cuh) and of the walk records
     const int world = sh ? sh->world : 1;
@@ -618,7 +618,7 @@ static int solve_device(int n, R* x_user, const int* nbd, const R* l, const R* u
     }
     if (!done) {
       const bool fused = hs.cnstnd != 0;
-      const int g_walk = walk_coop_grid<R, H, S>();
+      const int g_walk = walk_coop_grid<R, H, S>(true);
       auto round = [&]() {
         k_round_begin<R, H, S><<<1, 32, 0, stream>>>(c);
         c.stages = p.gcp.stages;

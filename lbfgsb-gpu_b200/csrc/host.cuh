@@ -258,16 +258,23 @@ static void walk_buffers(Workspace<R, H, S>& w, Ctx<R, H, S>& c, size_t N) {
   c.wsc = reinterpret_cast<WalkScratch*>(w.template alloc<unsigned char>(walk_scratch_bytes<S>((int)N)));
 }
 
-// Grid of the cooperative walk: CTAs that are all resident at once (one per SM at most).
+// Grid of the cooperative walk: CTAs that are all resident at once (one per SM at most).  A
+// host-driven solve launches it only when a walk is due, on every SM.  A device-driven round
+// launches it always, nearly always to return at once, and takes half the SMs: a CTA holds most
+// of an SM's shared memory, and a grid of all SMs waits until no other solve's CTA is left on any,
+// which lets solves on several threads run only one after another.  us a solve, 8 threads,
+// 148 / 74 / 64 CTAs: n = 64^2 FP64 722 / 468 / 476, 256^2 FP32 1122 / 802 / 791, 1024^2 FP64
+// 3644 / 3233 / 3245; a walk of 1.7 million breakpoints (n = 1024^2), one thread: 55.6 / 60.9 / 62.4
+// ms, of 426,000: 14.3 / 14.8 / 14.9.
 template <typename R, typename H, typename S>
-static int walk_coop_grid() {
+static int walk_coop_grid(bool every_round) {
   int per_sm = 0;
   CK(cudaFuncSetAttribute(k_walk_coop<R, H, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                           (int)sizeof(WalkCoop<S>)));
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk_coop<R, H, S>, kWalkThreads,
                                                    sizeof(WalkCoop<S>)));
   if (per_sm < 1) throw CudaFailure{cudaErrorCooperativeLaunchTooLarge, "k_walk_coop occupancy", __LINE__};
-  return device_sms();
+  return every_round ? std::max(1, device_sms() / 2) : device_sms();
 }
 
 // The cooperative walk: listing, selection and walk in one launch whose CTAs are
