@@ -79,3 +79,30 @@ def test_ended_instances_before_a_failure_are_delivered(mark):
         else:
             assert stat[k] != 0
             np.testing.assert_array_equal(x[k], np.float32(0.25))
+
+
+def test_large_and_small_instances_come_back():
+    """Instances on both sides of the size from which x is copied back on its own (2^21)."""
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import lbfgsb_b200 as LB
+    sides = [1449, 40, 1448]  # 1448^2 < 2^21 < 1449^2
+    opt = LB.default_option(np.float32)
+    opt.eps_f = opt.eps_g = opt.eps_x = 0.0
+    opt.max_iteration = 3
+
+    def solve(ids):
+        bt = LB.SynthBatch(sides, [3, 4, 5])
+        xs = [torch.full((sides[p] ** 2,), 0.25, dtype=torch.float32, device="cuda") for p in ids]
+        rc, stat, summ, _ = LB.solve_batch_device(bt, xs, opt, ids=ids)
+        torch.cuda.synchronize()
+        assert rc == 0 and stat == [0] * len(ids)
+        bt.close()
+        return xs, [(s.info, s.num_iteration, s.residual_g) for s in summ]
+
+    mixed, summ = solve([0, 1, 2])
+    for k in range(3):
+        alone, s = solve([k])
+        assert s[0] == summ[k] and not torch.equal(mixed[k], torch.full_like(mixed[k], 0.25))
+        assert torch.equal(alone[0], mixed[k])
