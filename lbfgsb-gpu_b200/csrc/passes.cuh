@@ -691,7 +691,7 @@ __device__ __forceinline__ void freev_formk_pass(const Ctx<R, H, S>& c, CtaPos c
   // [8..15] sum_F s_j y_col in registers; sum_A s_col s_j and sum_A s_col y_j per thread in
   // shared memory after the stage ring (entry q of thread e at nra[(q / 4) * CONS + e],
   // component q % 4), which keeps the thread within the register file's share of a
-  // 17-warp CTA
+  // 18-warp CTA
   A nrow[kOneRole ? 2 * kMaxM : 1];
 #pragma unroll
   for (int k = 0; k < (kOneRole ? 2 * kMaxM : 1); k++) nrow[k] = A(0);

@@ -13,9 +13,10 @@
 //            key order with the reference's recurrence for f', f'', c and p.
 // Two forms: k_walk_coop (single-instance solves) lists, selects, sorts and prepares with the
 // whole grid, a cooperative launch with a bounded grid barrier, and walks in CTA 0 as a
-// pipeline of warps; k_walk (one CTA per instance, used by batched solves, with k_walk_gather
-// before it) does everything in one CTA as described above.  Breakpoints with equal t are passed in increasing variable index (the heap's order
-// among exact ties is an artefact of its layout).
+// pipeline of warps; walk_pass (batched solves: kb_walk, one CTA per instance, after
+// kb_walk_gather) does everything in one CTA as described above.  Breakpoints with equal t are
+// passed in increasing variable index (the heap's order among exact ties is an artefact of its
+// layout).
 #pragma once
 
 #include "common.cuh"
@@ -340,7 +341,7 @@ __device__ __forceinline__ void walk_end(DevState<S>* st, WalkCarry<S>& w, S* wo
   st->gcp_state = GCP_DONE;
 }
 
-// The whole walk in one CTA (batched solves: one CTA per instance, after k_walk_gather).
+// The whole walk in one CTA (batched solves: one CTA per instance, after kb_walk_gather).
 template <typename R, typename H, typename S>
 __device__ __forceinline__ void walk_pass(const Ctx<R, H, S>& c, const R* __restrict__ x,
                                           const R* __restrict__ g) {
@@ -443,11 +444,6 @@ __device__ __forceinline__ void walk_pass(const Ctx<R, H, S>& c, const R* __rest
   if (threadIdx.x != 0) return;
   if (sm.done == 2) return;  // a failed M*wbp: the driver resets the memory
   walk_end(st, w, sm.work[0]);
-}
-template <typename R, typename H, typename S>
-__global__ void __launch_bounds__(kWalkThreads) k_walk(Ctx<R, H, S> c, const R* __restrict__ x,
-                                                       const R* __restrict__ g) {
-  walk_pass<R, H, S>(c, x, g);
 }
 
 // ---- the cooperative walk of single-instance solves ------------------------------------
