@@ -482,7 +482,8 @@ int lbfgsb_b200_copy(void* dst, const void* src, size_t bytes, int kind);
  * and the value the solver reports as summary.residual_g; x, g, nbd, l, u are device
  * arrays of length n.  Enqueued on `stream`, nothing is synchronised.  It calls no
  * allocator: its scratch is a static 64 KB device array, so n is limited to
- * 0..33554432 (8192 per-CTA maxima of 4096 variables); a larger n returns
+ * 0..33554432 (8192 per-CTA maxima of 4096 variables; x, l and u are read only for the
+ * variables whose nbd has the bound); a larger n returns
  * LBFGSB_B200_ERR_ARGUMENT with a message in lbfgsb_b200_last_error().  Meant for callers
  * that must not allocate, such as the solver's callbacks, which run in the middle of its
  * stream work.  Every call on a device shares the scratch: calls that overlap on the GPU

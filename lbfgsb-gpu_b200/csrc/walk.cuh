@@ -488,7 +488,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned int& ta
 // What bounds it: f', four dependent additions of 8.3 cycles each, 33-40 cycles a key; with the
 // chunk's selection, sort and preparation (40-60 us for 8192 keys) a key takes 35 ns.  One
 // thread walking key by key, with 64 rows of M*wbp prepared at a time by 64 threads, took
-// 0.46-0.52 us a key (n = 512^2, a solve with 426,000 keys in six walks: 190.7 -> 15.1 ms); f'
+// 0.46-0.52 us a key (n = 512^2, a solve with 426,000 keys in six walks: 190.7 -> 14.6 ms); f'
 // and f'' on one thread, and f' with its loads waited for, took 74-84 cycles a key (23.2 ms).
 constexpr int kWalkRows = 8192;       // breakpoints of a chunk at most
 constexpr int kWalkFirst = 1024;      // of the first chunk (most walks are short); then doubled
